@@ -82,7 +82,7 @@ def listed():
              steps=4),
         # the adjoint configuration: 200 steps of 1e6 parcels, checkpoints every 20
         dict(name="adjoint_hex128_mixed", kind="adjoint", nx=128, ny=128, nz=128,
-             parcels=1_000_000, precision="mixed", steps=200, checkpoint=20),
+             parcels=1_000_000, precision="mixed", steps=200, checkpoint=20, sort=20),
     ]
 
 
@@ -128,7 +128,7 @@ def draw(rng):
                     substeps=sub, sort=rng.choice([0, 20]), steps=rng.choice([1, 4]))
     return dict(kind=kind, **box, parcels=_log(rng, 1_000, 800_000),
                 precision=rng.choice(["mixed", "mixed", "fp64"]), steps=rng.choice([20, 50, 130]),
-                checkpoint=rng.choice([7, 10, 20]))
+                checkpoint=rng.choice([7, 10, 20]), sort=rng.choice([0, 20]))
 
 
 def fluid_factor(k):
