@@ -55,7 +55,7 @@ enum {
 };
 enum {
     ST_DEPOSIT_DETERMINISTIC = 0, /* warp-aggregated fixed-point sums: bitwise reproducible */
-    ST_DEPOSIT_ATOMIC = 1         /* one FP64 atomicAdd per deposit (A:714-725 in FP64)     */
+    ST_DEPOSIT_ATOMIC = 1         /* FP64 atomicAdd (A:714-725 in FP64) of warp run sums      */
 };
 
 /* Uniform cuboid mesh, cells numbered x fastest (A:222-270, A:684-691). */

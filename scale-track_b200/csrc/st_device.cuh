@@ -141,9 +141,9 @@ struct Quant {
     float thr_small; /* 2^(SMALL_Q_BITS+L) as float when that is a normal float, else 0 */
 };
 
-/* Quantised deposits below 2^SMALL_Q_BITS in magnitude: a sum of up to four of them fits in
+/* Quantised deposits below 2^SMALL_Q_BITS in magnitude: a sum of up to eight of them fits in
  * a 32-bit integer (the warp run reduction's 32-bit path). */
-constexpr int SMALL_Q_BITS = 29;
+constexpr int SMALL_Q_BITS = 28;
 
 __device__ __forceinline__ Quant make_quant(int L, int cap)
 {
@@ -222,6 +222,21 @@ __device__ __forceinline__ void quantize3(const double d[3], const Quant& qp, do
     for (int k = 0; k < 3; ++k) q[k] = quantize(d[k], qp, amax, ovf);
 }
 
+/* Reductions without a return value into global memory.  Spelled out in PTX: where the
+ * accumulator's address comes from a descriptor in memory (several clouds in one launch) the
+ * compiler sees a generic pointer and issues atomics that return the old value, which each
+ * warp then waits for. */
+__device__ __forceinline__ void red_add(unsigned long long* p, unsigned long long v)
+{
+    asm volatile("red.global.add.u64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "l"(v)
+                 : "memory");
+}
+__device__ __forceinline__ void red_add(double* p, double v)
+{
+    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"(v)
+                 : "memory");
+}
+
 template <int DEP, class V>
 __device__ __forceinline__ void deposit_direct(const V dep[3], int64_t cell0,
                                                unsigned long long* acc, double* src,
@@ -230,15 +245,15 @@ __device__ __forceinline__ void deposit_direct(const V dep[3], int64_t cell0,
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         if (DEP == DEP_ATOMIC) {
-            if (dep[c] != (V)0) atomicAdd(src + 3 * cell0 + c, (double)dep[c]);
+            if (dep[c] != (V)0) red_add(src + 3 * cell0 + c, (double)dep[c]);
         } else {
             long long q = quantize(dep[c], qp, amax, ovf);
             if (DEP == DEP_DET1) {
-                if (q) atomicAdd(acc + 3 * cell0 + c, (unsigned long long)q);
+                if (q) red_add(acc + 3 * cell0 + c, (unsigned long long)q);
             } else if (DEP == DEP_DET2) {
                 if (q) {
-                    atomicAdd(acc + 2 * (3 * cell0 + c), (unsigned long long)(q >> 32));
-                    atomicAdd(acc + 2 * (3 * cell0 + c) + 1,
+                    red_add(acc + 2 * (3 * cell0 + c), (unsigned long long)(q >> 32));
+                    red_add(acc + 2 * (3 * cell0 + c) + 1,
                               (unsigned long long)q & 0xffffffffULL);
                 }
             }
@@ -246,19 +261,21 @@ __device__ __forceinline__ void deposit_direct(const V dep[3], int64_t cell0,
     }
 }
 
-#ifndef ST_SCAN_STEPS
-#define ST_SCAN_STEPS 2
-#endif
-constexpr int SCAN_STEPS = ST_SCAN_STEPS;   /* 0..5 */
-constexpr int SPAN = 1 << SCAN_STEPS;        /* lanes summed per emitted chunk */
+/* Steps of the run scan: it sums chunks of 2^steps lanes.  Three steps halve the adds of runs
+ * of five to eight parcels against two (a freshly sorted cloud of five parcels per cell); with
+ * two limbs a step costs twelve more shuffles, and two steps are faster (FP64, 2e6 parcels on
+ * 97 x 64 x 53 cells: 74 us per launch with two steps, 79 us with three and the hand-over of
+ * emit_runs). */
+template <int DEP>
+constexpr int scan_steps = DEP == DEP_DET2 ? 2 : 3;
 
-/* Inclusive scan over the lane's run of equal keys, limited to SPAN lanes (runs are
+/* Inclusive scan over the lane's run of equal keys, limited to 2^STEPS lanes (runs are
  * contiguous lane ranges). */
-template <class T>
+template <int STEPS, class T>
 __device__ __forceinline__ T seg_scan(T v, int lane, int segstart)
 {
 #pragma unroll
-    for (int off = 1; off < SPAN; off <<= 1) {
+    for (int off = 1; off < (1 << STEPS); off <<= 1) {
         T t = __shfl_up_sync(FULL_MASK, v, off);
         if (lane - off >= segstart) v += t;
     }
@@ -291,13 +308,57 @@ __device__ __forceinline__ T ld_stream(const T* p) { return ld_stream_(p); }
 template <class T>
 __device__ __forceinline__ void st_stream(T* p, T v) { __stcs(p, v); }
 
+/* 8-byte words of shared memory that one warp's deposit_warp needs (its last argument): up to
+ * 96 sums and the 32 cells they go to. */
+template <int DEP, class V>
+constexpr int dep_ws_words = DEP == DEP_ATOMIC                  ? 96 + 16
+                             : DEP == DEP_DET1 && sizeof(V) == 4 ? 48 + 16
+                                                                 : 1;
+
+/* Writes a warp's run sums out: the lanes with `out` hold three values each (v) for the three
+ * consecutive words at dst + 3 * key.  The values are handed over through shared memory so
+ * that consecutive lanes add to consecutive words: the words of one cell, and of neighbouring
+ * cells, go out in one instruction and merge into few 32-byte sectors, where one instruction
+ * per component sends every value as a request of its own.  The adds were what bound the hex
+ * step once parcels have drifted from their sorted order (1e7 parcels on 128^3 cells, mean of
+ * a re-sort cycle of 20 steps, conversion in stream order: 209 us per launch, 146 us with the
+ * adds left out, 186 us with this hand-over and the longer chunks of scan_steps). */
+template <class T, class W>
+__device__ __forceinline__ void emit_runs(bool out, int32_t key, const T v[3], W* dst,
+                                          unsigned long long* ws, int lane)
+{
+    const unsigned outs = __ballot_sync(FULL_MASK, out);
+    T* const sv = reinterpret_cast<T*>(ws);
+    int32_t* const sk = reinterpret_cast<int32_t*>(sv + 96);
+    if (out) {
+        const int r = __popc(outs & ((1u << lane) - 1u));
+#pragma unroll
+        for (int k = 0; k < 3; ++k) sv[3 * r + k] = v[k];
+        sk[r] = key;
+    }
+    __syncwarp();
+    const int items = 3 * __popc(outs);
+    for (int i = lane; i < items; i += 32) {
+        const int r = (int)((unsigned)i / 3u);
+        const T q = sv[i];
+        if (q != (T)0) {
+            W* const p = dst + 3 * (int64_t)sk[r] + (i - 3 * r);
+            if constexpr (sizeof(T) == 4) red_add(p, (W)(long long)q);
+            else red_add(p, (W)q);
+        }
+    }
+    __syncwarp();
+}
+
 /* Final deposits of 32 consecutive parcels (one per lane, key < 0 = none): runs of equal
- * cells are summed with a segmented warp scan and the last lane of each run adds the sum. */
+ * cells are summed with a segmented warp scan and the last lane of each run adds the sum.
+ * The FP64 atomic mode sums its runs in FP64 the same way.
+ * `ws`: this warp's dep_ws_words<DEP, V> words of shared memory. */
 template <int DEP, class V>
 __device__ __forceinline__ void deposit_warp(int32_t key, const V dep[3],
                                              unsigned long long* acc, double* src,
                                              const Quant& qp, int lane, AmaxT<V>& amax,
-                                             unsigned& ovf)
+                                             unsigned& ovf, unsigned long long* ws)
 {
     if (DEP == DEP_PROBE) {
         if (key >= 0) {
@@ -306,19 +367,18 @@ __device__ __forceinline__ void deposit_warp(int32_t key, const V dep[3],
         }
         return;
     }
-    if (DEP == DEP_ATOMIC) {
-        if (key >= 0) deposit_direct<DEP_ATOMIC, V>(dep, key, acc, src, qp, amax, ovf);
-        return;
-    }
+    constexpr int STEPS = scan_steps<DEP>, SPAN = 1 << STEPS;
     const int prev = __shfl_up_sync(FULL_MASK, key, 1);
     const bool head = (lane == 0) || (prev != key);
     const unsigned heads = __ballot_sync(FULL_MASK, head);
+    /* quantised deposits, and whether the 32-bit path holds for every lane */
+    int q32[3] = {0, 0, 0};
+    bool narrow = false;
     if constexpr (DEP == DEP_DET1 && sizeof(V) == 4) {
         /* 32-bit path: when every lane's deposit components quantise below 2^SMALL_Q_BITS
          * (|d0| + |d1| + |d2| below 2^(SMALL_Q_BITS+L), the bound argument of quantize3), the
-         * integers are those of quantize3, a chunk of SPAN <= 4 lanes sums below 2^31, and the
+         * integers are those of quantize3, a chunk of SPAN <= 8 lanes sums below 2^31, and the
          * run sums are formed in 32-bit registers: the same integers reach the accumulators. */
-        int q32[3] = {0, 0, 0};
         bool small = key < 0;
         if (key >= 0) {
             const float a0 = fabsf((float)dep[0]), a1 = fabsf((float)dep[1]),
@@ -330,50 +390,34 @@ __device__ __forceinline__ void deposit_warp(int32_t key, const V dep[3],
                 small = true;
             }
         }
-        static_assert(SPAN <= 4, "32-bit chunk sums");
-        if (__all_sync(FULL_MASK, small)) {
-            if (heads == 1u) {
-                /* one cell for the whole warp: 16-bit halves, each sum exact in 32 bits */
-                if (key >= 0) {
-                    long long t[3];
+        static_assert(SMALL_Q_BITS + STEPS <= 31, "32-bit chunk sums");
+        narrow = __all_sync(FULL_MASK, small);
+        if (narrow && heads == 1u) {
+            /* one cell for the whole warp: 16-bit halves, each sum exact in 32 bits */
+            if (key >= 0) {
+                long long t[3];
 #pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        const int shi = __reduce_add_sync(FULL_MASK, q32[k] >> 16);
-                        const unsigned slo = __reduce_add_sync(FULL_MASK, (unsigned)q32[k] & 0xffffu);
-                        t[k] = (long long)shi * 65536LL + (long long)slo;
-                    }
-                    if (lane == 0) {
-                        unsigned long long* p = acc + 3 * (int64_t)key;
-#pragma unroll
-                        for (int k = 0; k < 3; ++k)
-                            if (t[k]) atomicAdd(p + k, (unsigned long long)t[k]);
-                    }
+                for (int k = 0; k < 3; ++k) {
+                    const int shi = __reduce_add_sync(FULL_MASK, q32[k] >> 16);
+                    const unsigned slo = __reduce_add_sync(FULL_MASK, (unsigned)q32[k] & 0xffffu);
+                    t[k] = (long long)shi * 65536LL + (long long)slo;
                 }
-                return;
-            }
-            const int segstart = 31 - __clz(heads & (FULL_MASK >> (31 - lane)));
-            const bool tail = (lane == 31) || ((heads >> (lane + 1)) & 1u);
-            const unsigned tails = __ballot_sync(FULL_MASK, tail);
-            const int tailpos = lane + __ffs(tails >> lane) - 1;
-            const bool emit = ((tailpos - lane) & (SPAN - 1)) == 0;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) q32[k] = seg_scan(q32[k], lane, segstart);
-            if (emit && key >= 0) {
-                unsigned long long* p = acc + 3 * (int64_t)key;
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    if (q32[k]) atomicAdd(p + k, (unsigned long long)(long long)q32[k]);
+                const long long mine = lane == 0 ? t[0] : (lane == 1 ? t[1] : t[2]);
+                if (lane < 3 && mine)
+                    red_add(acc + 3 * (int64_t)key + lane, (unsigned long long)mine);
             }
             return;
         }
     }
     long long q[3] = {0, 0, 0};
-    if (key >= 0) quantize3(dep, qp, amax, ovf, q);
-    if (DEP == DEP_DET1 && heads == 1u) {
+    if constexpr (DEP != DEP_ATOMIC) {
+        if (!narrow && key >= 0) quantize3(dep, qp, amax, ovf, q);
+    }
+    if (DEP == DEP_DET1 && !narrow && heads == 1u) {
         /* One cell for the whole warp (dense cells after a re-sort): exact full-warp
-         * reductions replace the scan and lane 0 adds the sum.  With q = hi*2^32 + lo, the
-         * sums of lo's two 16-bit halves stay below 2^21, and |sum of hi| <= 2^30 + 32 because
-         * the headroom bounds the magnitudes of all of a step's deposits together by 2^62. */
+         * reductions replace the scan.  With q = hi*2^32 + lo, the sums of lo's two 16-bit
+         * halves stay below 2^21, and |sum of hi| <= 2^30 + 32 because the headroom bounds
+         * the magnitudes of all of a step's deposits together by 2^62. */
         if (key >= 0) {
             long long t[3];
 #pragma unroll
@@ -384,46 +428,54 @@ __device__ __forceinline__ void deposit_warp(int32_t key, const V dep[3],
                 const unsigned s1 = __reduce_add_sync(FULL_MASK, lo >> 16);
                 t[k] = shi * 4294967296LL + (long long)s0 + (long long)s1 * 65536LL;
             }
-            if (lane == 0) {
-                unsigned long long* p = acc + 3 * (int64_t)key;
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    if (t[k]) atomicAdd(p + k, (unsigned long long)t[k]);
-            }
+            const long long mine = lane == 0 ? t[0] : (lane == 1 ? t[1] : t[2]);
+            if (lane < 3 && mine)
+                red_add(acc + 3 * (int64_t)key + lane, (unsigned long long)mine);
         }
         return;
     }
-    const int segstart = 31 - __clz(heads & (FULL_MASK >> (31 - lane)));
-    const bool tail = (lane == 31) || ((heads >> (lane + 1)) & 1u);
-    /* A scan of SCAN_STEPS steps sums runs in chunks of SPAN lanes: lane j holds the sum of
+    /* A scan of STEPS steps sums runs in chunks of SPAN lanes: lane j holds the sum of
      * [max(run start, j - SPAN + 1), j]; the run's last lane and every SPAN-th lane before it
      * add their chunk, which covers the run exactly once. */
+    const int segstart = 31 - __clz(heads & (FULL_MASK >> (31 - lane)));
+    const bool tail = (lane == 31) || ((heads >> (lane + 1)) & 1u);
     const unsigned tails = __ballot_sync(FULL_MASK, tail);
     const int tailpos = lane + __ffs(tails >> lane) - 1;
-    const bool emit = ((tailpos - lane) & (SPAN - 1)) == 0;
-    if (DEP == DEP_DET1) {
+    const bool out = ((tailpos - lane) & (SPAN - 1)) == 0 && key >= 0;
+    if constexpr (DEP == DEP_ATOMIC) {
+        double t[3];
 #pragma unroll
-        for (int k = 0; k < 3; ++k) q[k] = seg_scan(q[k], lane, segstart);
-        if (emit && key >= 0) {
+        for (int k = 0; k < 3; ++k) t[k] = seg_scan<STEPS>((double)dep[k], lane, segstart);
+        emit_runs(out, key, t, src, ws, lane);
+    } else if constexpr (DEP == DEP_DET1) {
+        if (narrow) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) q32[k] = seg_scan<STEPS>(q32[k], lane, segstart);
+            emit_runs(out, key, q32, acc, ws, lane);
+            return;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) q[k] = seg_scan<STEPS>(q[k], lane, segstart);
+        if (out) {   /* a warp with a large deposit, or FP32 deposits outside the fast range */
             unsigned long long* p = acc + 3 * (int64_t)key;
 #pragma unroll
             for (int k = 0; k < 3; ++k)
-                if (q[k]) atomicAdd(p + k, (unsigned long long)q[k]);
+                if (q[k]) red_add(p + k, (unsigned long long)q[k]);
         }
     } else {
         long long hi[3];
         unsigned long long lo[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            hi[k] = seg_scan(q[k] >> 32, lane, segstart);
-            lo[k] = seg_scan((unsigned long long)q[k] & 0xffffffffULL, lane, segstart);
+            hi[k] = seg_scan<STEPS>(q[k] >> 32, lane, segstart);
+            lo[k] = seg_scan<STEPS>((unsigned long long)q[k] & 0xffffffffULL, lane, segstart);
         }
-        if (emit && key >= 0) {
+        if (out) {
             unsigned long long* p = acc + 6 * (int64_t)key;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                if (hi[k]) atomicAdd(p + 2 * k, (unsigned long long)hi[k]);
-                if (lo[k]) atomicAdd(p + 2 * k + 1, lo[k]);
+                if (hi[k]) red_add(p + 2 * k, (unsigned long long)hi[k]);
+                if (lo[k]) red_add(p + 2 * k + 1, lo[k]);
             }
         }
     }

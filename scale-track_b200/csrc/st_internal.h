@@ -28,6 +28,10 @@ constexpr int QUANT_GROWTH_BITS = 8;   /* deposits may grow 2^8 x between steps 
 
 enum DepMode { DEP_DET1 = 0, DEP_DET2 = 1, DEP_ATOMIC = 2, DEP_PROBE = 3 };
 
+/* The deterministic deposit of a precision: one limb for FP32 velocities, two for FP64. */
+template <class V>
+constexpr int det_mode = sizeof(V) == 8 ? DEP_DET2 : DEP_DET1;
+
 /* Mixed precision: FP64 positions with FP32 drag and velocities. */
 template <class P, class V>
 constexpr bool is_mixed = sizeof(P) == 8 && sizeof(V) == 4;

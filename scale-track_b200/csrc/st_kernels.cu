@@ -79,6 +79,8 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     constexpr bool DET = (DEP == DEP_DET1 || DEP == DEP_DET2);
 
+    __shared__ unsigned long long dep_ws[8][dep_ws_words<DEP, V>];
+    unsigned long long* const ws = dep_ws[threadIdx.x >> 5];
     if (!ONE) {   /* the table of x^0.687 serves the multi-substep loop */
         pow_tab_fill();
         __syncthreads();
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
                     st_stream(cl.w + i, vel[2]);
                 }
             }
-            deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf);
+            deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf, ws);
         }
     }
     if (cur >= 0) flush_ctl<DEP>(a.ctl + cur, lane, amax, ovf, nlost);
@@ -207,8 +209,7 @@ static cudaError_t launch_step_t(const StepArgs<P, V>& a, int dep, int grid, int
                                  cudaStream_t s)
 {
     switch (dep) {
-    case DEP_DET1: k_step<P, V, DEP_DET1, ONE, SINGLE><<<grid, block, 0, s>>>(a); break;
-    case DEP_DET2: k_step<P, V, DEP_DET2, ONE, SINGLE><<<grid, block, 0, s>>>(a); break;
+    case det_mode<V>: k_step<P, V, det_mode<V>, ONE, SINGLE><<<grid, block, 0, s>>>(a); break;
     case DEP_ATOMIC: k_step<P, V, DEP_ATOMIC, ONE, SINGLE><<<grid, block, 0, s>>>(a); break;
     case DEP_PROBE: k_step<P, V, DEP_PROBE, ONE, SINGLE><<<grid, block, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;
@@ -232,8 +233,7 @@ static int max_active_t(int dep, int block)
     int nb = 0;
     cudaError_t e = cudaErrorInvalidValue;
     switch (dep) {
-    case DEP_DET1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step<P, V, DEP_DET1, ONE, SINGLE>, block, 0); break;
-    case DEP_DET2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step<P, V, DEP_DET2, ONE, SINGLE>, block, 0); break;
+    case det_mode<V>: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step<P, V, det_mode<V>, ONE, SINGLE>, block, 0); break;
     case DEP_ATOMIC: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step<P, V, DEP_ATOMIC, ONE, SINGLE>, block, 0); break;
     case DEP_PROBE: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step<P, V, DEP_PROBE, ONE, SINGLE>, block, 0); break;
     default: break;

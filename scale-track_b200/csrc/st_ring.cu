@@ -52,7 +52,8 @@ __device__ __forceinline__ void ring_slices(const StepArgs<P, V>& a, P* xs, P* y
                                             V* vs, V* ws, const V* ds, int j0, int64_t nvalid,
                                             unsigned long long* acc, double* src,
                                             const Quant& qp, int lane, AmaxT<V>& amax,
-                                            unsigned& ovf, unsigned& nlost)
+                                            unsigned& ovf, unsigned& nlost,
+                                            unsigned long long* scr)
 {
     P X[RING_SPW], Y[RING_SPW], Z[RING_SPW];
     V Uv[RING_SPW], Vv[RING_SPW], Wv[RING_SPW], D[RING_SPW];
@@ -111,7 +112,7 @@ __device__ __forceinline__ void ring_slices(const StepArgs<P, V>& a, P* xs, P* y
                 ring_st<GLOBAL>(ws + j, vel[2]);
             }
         }
-        deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf);
+        deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf, scr);
     }
 }
 
@@ -126,11 +127,12 @@ struct HexRing {
     AmaxT<V>& amax;
     unsigned& ovf;
     unsigned& nlost;
+    unsigned long long* scr;
     template <bool GLOBAL>
     __device__ __forceinline__ void run(const RingArrays<P, V>& r, int j0, int64_t nvalid)
     {
         ring_slices<P, V, DEP, ONE, GLOBAL>(a, r.x, r.y, r.z, r.u, r.v, r.w, r.d, j0, nvalid, acc,
-                                            src, qp, lane, amax, ovf, nlost);
+                                            src, qp, lane, amax, ovf, nlost, scr);
     }
 };
 
@@ -145,9 +147,10 @@ __global__ void __launch_bounds__(HexShapeOf<V>::type::THREADS, 1)
     AmaxT<V> amax = (V)0;
     unsigned ovf = 0, nlost = 0;
     const int lane = threadIdx.x & 31;
+    __shared__ unsigned long long dep_ws[HexShape::CONS][dep_ws_words<DEP, V>];
     HexRing<P, V, DEP, ONE> step{a, DET ? a.one.acc : nullptr,
                                  DEP == DEP_ATOMIC ? a.one.src : nullptr, qp, lane, amax, ovf,
-                                 nlost};
+                                 nlost, dep_ws[min(threadIdx.x >> 5, HexShape::CONS - 1)]};
     if (!ONE) pow_tab_fill();   /* ring_block synchronises the block before any step */
     ring_emax_init();
     if (!ring_block<HexShape, P, V, false>(a.one, a.ctl, step, a.wait_cycles)) return;
@@ -196,8 +199,8 @@ static cudaError_t launch_ring_t(const StepArgs<P, V>& a, int nsm, cudaStream_t 
 template <class P, class V>
 cudaError_t ring_prepare()
 {
-    const cudaError_t r[6] = {ring_attr<P, V, DEP_DET1, true>(), ring_attr<P, V, DEP_DET1, false>(),
-                              ring_attr<P, V, DEP_DET2, true>(), ring_attr<P, V, DEP_DET2, false>(),
+    constexpr int DET = det_mode<V>;
+    const cudaError_t r[4] = {ring_attr<P, V, DET, true>(), ring_attr<P, V, DET, false>(),
                               ring_attr<P, V, DEP_ATOMIC, true>(),
                               ring_attr<P, V, DEP_ATOMIC, false>()};
     for (cudaError_t e : r)
@@ -209,7 +212,7 @@ template <class P, class V>
 bool ring_eligible(const StepArgs<P, V>& a, int dep)
 {
     if (a.nclouds != 1 || a.one.n <= 0) return false;
-    if (dep != DEP_DET1 && dep != DEP_DET2 && dep != DEP_ATOMIC) return false;
+    if (dep != det_mode<V> && dep != DEP_ATOMIC) return false;
     const void* p[7] = {a.one.x, a.one.y, a.one.z, a.one.u, a.one.v, a.one.w, a.one.d};
     for (const void* q : p)
         if (reinterpret_cast<uintptr_t>(q) % 16) return false;
@@ -222,10 +225,8 @@ cudaError_t launch_step_ring(const StepArgs<P, V>& a, int dep, int nsm, cudaStre
     if (a.nclouds != 1) return cudaErrorInvalidValue;
     const bool one = a.phys.nsub == 1;
     switch (dep) {
-    case DEP_DET1: return one ? launch_ring_t<P, V, DEP_DET1, true>(a, nsm, s)
-                              : launch_ring_t<P, V, DEP_DET1, false>(a, nsm, s);
-    case DEP_DET2: return one ? launch_ring_t<P, V, DEP_DET2, true>(a, nsm, s)
-                              : launch_ring_t<P, V, DEP_DET2, false>(a, nsm, s);
+    case det_mode<V>: return one ? launch_ring_t<P, V, det_mode<V>, true>(a, nsm, s)
+                                 : launch_ring_t<P, V, det_mode<V>, false>(a, nsm, s);
     case DEP_ATOMIC: return one ? launch_ring_t<P, V, DEP_ATOMIC, true>(a, nsm, s)
                                 : launch_ring_t<P, V, DEP_ATOMIC, false>(a, nsm, s);
     default: return cudaErrorInvalidValue;

@@ -326,6 +326,8 @@ __global__ void __launch_bounds__(256, TetMinBlocks<V>::value) k_step_tet(const 
     unsigned ovf = 0, nlost = 0;
     const int nsub = ONE ? 1 : ph.nsub;
     const bool count_hops = a.hop_hist != nullptr && DEP != DEP_PROBE;
+    __shared__ unsigned long long dep_ws[8][dep_ws_words<DEP, V>];
+    unsigned long long* const ws = dep_ws[threadIdx.x >> 5];
     if (threadIdx.x < 8) s_tet_hist[threadIdx.x] = 0;
     __syncthreads();
 
@@ -368,7 +370,7 @@ __global__ void __launch_bounds__(256, TetMinBlocks<V>::value) k_step_tet(const 
                 st_stream(cl->cell + i, cell);
             }
         }
-        deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf);
+        deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf, ws);
         }
     }
     if (cur_cloud >= 0) flush_ctl<DEP>(a.ctl + cur_cloud, lane, amax, ovf, nlost);
@@ -398,6 +400,7 @@ struct TetRing {
     AmaxT<V>& amax;
     unsigned& ovf;
     unsigned& nlost;
+    unsigned long long* ws;
     template <bool GLOBAL>
     __device__ __forceinline__ void run(const RingArrays<double, V>& r, int j0, int64_t nvalid)
     {
@@ -430,7 +433,7 @@ struct TetRing {
                     ring_st<GLOBAL>(r.cell + j, cell);
                 }
             }
-            deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf);
+            deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf, ws);
         }
     }
 };
@@ -447,9 +450,11 @@ __global__ void __launch_bounds__(TetShape::THREADS, 1) k_step_tet_ring(const Te
     const bool count_hops = a.hop_hist != nullptr;
     if (threadIdx.x < 8) s_tet_hist[threadIdx.x] = 0;   /* ring_block synchronises */
     ring_emax_init();
+    __shared__ unsigned long long dep_ws[TetShape::CONS][dep_ws_words<DEP, V>];
     TetRing<V, DEP, ONE> step{a, DET ? a.one.acc : nullptr,
                               DEP == DEP_ATOMIC ? a.one.src : nullptr, qp, lane, count_hops,
-                              amax, ovf, nlost};
+                              amax, ovf, nlost,
+                              dep_ws[min(threadIdx.x >> 5, TetShape::CONS - 1)]};
     if (!ring_block<TetShape, double, V, true>(a.one, a.ctl, step, a.wait_cycles)) return;
     flush_ctl<DEP>(a.ctl, lane, amax, ovf, nlost, DEP != DEP_ATOMIC ? &s_ring_emax : nullptr);
     ring_consumers_sync<TetShape>();
@@ -493,7 +498,7 @@ template <class V>
 bool tet_ring_eligible(const TetStepArgs<V>& a, int dep)
 {
     if (a.nclouds != 1 || a.one.n <= 0 || !a.one.cell) return false;
-    if (dep != DEP_DET1 && dep != DEP_DET2 && dep != DEP_ATOMIC) return false;
+    if (dep != det_mode<V> && dep != DEP_ATOMIC) return false;
     const void* p[8] = {a.one.x, a.one.y, a.one.z, a.one.u, a.one.v, a.one.w, a.one.d, a.one.cell};
     for (const void* q : p)
         if (reinterpret_cast<uintptr_t>(q) % 16) return false;
@@ -505,10 +510,8 @@ cudaError_t launch_step_tet_ring(const TetStepArgs<V>& a, int dep, int nsm, cuda
 {
     const bool one = a.phys.nsub == 1;
     switch (dep) {
-    case DEP_DET1: return one ? launch_tet_ring_t<V, DEP_DET1, true>(a, nsm, s)
-                              : launch_tet_ring_t<V, DEP_DET1, false>(a, nsm, s);
-    case DEP_DET2: return one ? launch_tet_ring_t<V, DEP_DET2, true>(a, nsm, s)
-                              : launch_tet_ring_t<V, DEP_DET2, false>(a, nsm, s);
+    case det_mode<V>: return one ? launch_tet_ring_t<V, det_mode<V>, true>(a, nsm, s)
+                                 : launch_tet_ring_t<V, det_mode<V>, false>(a, nsm, s);
     case DEP_ATOMIC: return one ? launch_tet_ring_t<V, DEP_ATOMIC, true>(a, nsm, s)
                                 : launch_tet_ring_t<V, DEP_ATOMIC, false>(a, nsm, s);
     default: return cudaErrorInvalidValue;
@@ -520,8 +523,8 @@ cudaError_t launch_step_tet_ring(const TetStepArgs<V>& a, int dep, int nsm, cuda
 template <class V>
 cudaError_t tet_ring_prepare()
 {
-    const cudaError_t r[6] = {tet_ring_attr<V, DEP_DET1, true>(), tet_ring_attr<V, DEP_DET1, false>(),
-                              tet_ring_attr<V, DEP_DET2, true>(), tet_ring_attr<V, DEP_DET2, false>(),
+    constexpr int DET = det_mode<V>;
+    const cudaError_t r[4] = {tet_ring_attr<V, DET, true>(), tet_ring_attr<V, DET, false>(),
                               tet_ring_attr<V, DEP_ATOMIC, true>(),
                               tet_ring_attr<V, DEP_ATOMIC, false>()};
     for (cudaError_t e : r)
@@ -541,8 +544,7 @@ static cudaError_t launch_step_tet_t(const TetStepArgs<V>& a, int dep, int grid,
                                      cudaStream_t s)
 {
     switch (dep) {
-    case DEP_DET1: k_step_tet<V, DEP_DET1, ONE><<<grid, block, 0, s>>>(a); break;
-    case DEP_DET2: k_step_tet<V, DEP_DET2, ONE><<<grid, block, 0, s>>>(a); break;
+    case det_mode<V>: k_step_tet<V, det_mode<V>, ONE><<<grid, block, 0, s>>>(a); break;
     case DEP_ATOMIC: k_step_tet<V, DEP_ATOMIC, ONE><<<grid, block, 0, s>>>(a); break;
     case DEP_PROBE: k_step_tet<V, DEP_PROBE, ONE><<<grid, block, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;
@@ -563,8 +565,7 @@ static int tet_max_active_t(int dep, int block)
     int nb = 0;
     cudaError_t e = cudaErrorInvalidValue;
     switch (dep) {
-    case DEP_DET1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step_tet<V, DEP_DET1, ONE>, block, 0); break;
-    case DEP_DET2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step_tet<V, DEP_DET2, ONE>, block, 0); break;
+    case det_mode<V>: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step_tet<V, det_mode<V>, ONE>, block, 0); break;
     case DEP_ATOMIC: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step_tet<V, DEP_ATOMIC, ONE>, block, 0); break;
     case DEP_PROBE: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_step_tet<V, DEP_PROBE, ONE>, block, 0); break;
     default: break;
