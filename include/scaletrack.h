@@ -232,23 +232,24 @@ typedef struct st_tune_result {
  * changes positions, velocities or the fixed-point source. */
 ST_API int st_autotune(st_handle* h, double dt, int trial_steps, st_tune_result* out);
 
-/* Step kernel of a handle with one cloud (cuboid or tet mesh).  ST_STEP_KERNEL_RING (the
- * default): a persistent block per SM streams block tiles of 1024 parcels through a
+/* Step kernel of a handle with one cloud (cuboid or tet mesh).  ST_STEP_KERNEL_RING: a
+ * persistent block per SM streams block tiles of about a thousand parcels through a
  * shared-memory ring with bulk copies.  ST_STEP_KERNEL_WARP: every warp loads and steps its
- * own 32 parcels.  Both give bit-identical positions, velocities, cells, sources and walk
- * lengths; handles with several clouds, and the first (probe) pass of a run, always use the
- * warp kernel.  No counterpart in the
+ * own 32 parcels.  Without this call the library takes the faster one for the cloud's size,
+ * precision and substeps (the ring for large clouds).  Both give bit-identical positions,
+ * velocities, cells, sources and walk lengths; handles with several clouds, and the first
+ * (probe) pass of a run, always use the warp kernel.  No counterpart in the
  * reference (one kernel, A:1258-1269). */
 enum { ST_STEP_KERNEL_RING = 0, ST_STEP_KERNEL_WARP = 1 };
 ST_API int st_set_step_kernel(st_handle* h, int kind);
 /* With one cloud and the deterministic deposit, a step's conversion of the fixed-point sums
- * to the FP64 source (and the clearing of its accumulator) runs on a second stream of the
+ * to the FP64 source (and the clearing of its accumulator) may run on a second stream of the
  * library, concurrent with the next step on the handle's stream; the two steps use two
  * accumulators in turn.  st_get_source, st_synchronize and st_source_device order the
  * handle's stream after it, so work the caller enqueues on that stream afterwards sees the
- * source.  on = 0 runs the conversion in the handle's stream after each step instead (as
- * graph capture, several clouds, tet meshes, the sharded phases and the coupling shims always
- * do).  Results do not depend on the choice.  Default: on. */
+ * source.  on = 0 always runs the conversion in the handle's stream after each step (as small
+ * clouds, graph capture, several clouds, tet meshes, the sharded phases and the coupling
+ * shims do anyway).  Results do not depend on the choice.  Default: on. */
 ST_API int st_set_finalize_overlap(st_handle* h, int on);
 /* Failure detection of the ring step kernels: every wait of their shared-memory pipeline
  * (on a copy into a stage, or on the consumers releasing it) gives up after `cycles` SM clock

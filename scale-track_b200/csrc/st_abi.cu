@@ -13,8 +13,7 @@
  *   [probe + set_scale]   only on the first step after st_set_parcels or a new dt
  *   [zero source]         only in ST_DEPOSIT_ATOMIC mode
  *   step                  k_step: the parcel step and the warp-aggregated deposit
- *   finalize              fixed point -> FP64 source and next scale; then a memset clears
- *                         the accumulators
+ *   finalize              fixed point -> FP64 source, accumulators cleared, next scale
  *   [sort]                every sort_interval steps
  */
 #include <cstdarg>
@@ -144,7 +143,7 @@ struct st_handle {
     int steps_since_sort = 0;
     int block = 256;
     int grid = 0;
-    bool ring = true;      /* ST_STEP_KERNEL_RING for single-cloud steps */
+    int kernel = -1;       /* ST_STEP_KERNEL_* set by the caller, -1: use_ring's rule */
     int32_t* dexp = nullptr;   /* [nclouds] largest-deposit exponents of a sharded step */
     float* dsrc32 = nullptr;   /* when set, the finalize also writes the FP32 source here
                                   ([nclouds][stride]; the coupling's 4-byte exchange) */
@@ -482,6 +481,42 @@ int do_sort_all(st_handle* h)
     return ST_OK;
 }
 
+/* Programmatic dependent launch of the step's kernels: on the library's or a caller's own
+ * stream, outside graph capture (a captured graph keeps plain edges) and profiling (its events
+ * stand between the kernels).  It hides launch gaps of a few microseconds (1e4 parcels on 20^3
+ * cells: 13.0 -> 9.5 us per step, 1e5 on 32^3: 15.0 -> 12.3 us), so only handles with small
+ * accumulators use it: with large ones the waiting conversion takes SMs from other handles'
+ * steps (64 sources of 64^3 cells, three handles in turn: 1526 against 1358 us per step). */
+bool use_pdl(const st_handle* h)
+{
+    return (size_t)h->stride * h->p.n_clouds * h->limbs * 8 <= FINALIZE_CLEAR_BYTES &&
+           !h->capturing && !h->prof && h->stream != nullptr && h->stream != cudaStreamLegacy &&
+           h->stream != cudaStreamPerThread;
+}
+
+/* The ring or the per-warp kernel for a step of a single cloud of n parcels, unless the
+ * caller chose one.  A ring block works on whole tiles of about a thousand parcels, so a small
+ * cloud leaves SMs without a tile and the rest with one warp slice after another, while the
+ * per-warp kernel spreads every 32 parcels; the ring's bulk copies pay off once every block
+ * streams many tiles, and they do not pay when several substeps of arithmetic stand between a
+ * load and its store.  Measured, ring against per-warp kernel, us per step:
+ *   hex, FP32 and mixed:  1e4 15.9 / 9.5   1e5 14.6 / 12.3   1.5e6 41.1 / 41.0   4e6 84.5 / 92.6
+ *   hex, FP64:   1e5 17.7 / 15.0   4e5 25.2 / 24.9   5e5 30.1 / 32.1   4e6 141 / 151
+ *   hex, mixed, ten substeps:  1e6 118 / 99   4e6 386 / 333   1e7 987 / 859
+ *   tet, mixed:  2e5 23.0 / 21.5   4e5 29.0 / 29.4   1e6 47.5 / 50.2; three substeps:
+ *                2e5 37.7 / 35.9   1e6 80.5 / 87.3
+ *   tet, FP64:   4e5 35.6 / 35.8   7e5 64.6 / 64.4   1.5e6 105 / 108; three substeps:
+ *                1.5e6 190 / 186
+ * A wait limit set by the caller is about the ring's waits: the ring then runs at any size. */
+bool use_ring(const st_handle* h, int64_t n)
+{
+    if (h->kernel >= 0) return h->kernel == ST_STEP_KERNEL_RING;
+    if (h->wait_cycles != 0) return true;
+    const bool fp64 = h->p.precision == ST_PREC_FP64;
+    if (h->tet) return n >= (fp64 ? 1000000 : 300000);
+    return h->p.n_substeps == 1 && n >= (fp64 ? 450000 : 1500000);
+}
+
 /* Phases of one step.  PH_ALL is st_step.  A sharded step (one handle per rank, parcels
  * split over the ranks) runs PH_PROBE (first step only), PH_DEPOSIT and PH_FINISH as separate
  * calls, and the caller combines the ranks' exponents (max) and accumulators (sum) between
@@ -562,9 +597,8 @@ int step_phases(st_handle* h, double dt, int phase, bool empty, L&& launch, S&& 
         {
             ProfScope ps(h, ST_KERNEL_FINALIZE, h->fin_stream);
             CK(launch_finalize(h->limbs, acc_ovl, h->dsrc, h->dsrc32, h->dctl, Lf, h->dcounter,
-                               nc, h->stride, finalize_grid(h), h->fin_stream));
+                               nc, h->stride, finalize_grid(h), h->fin_stream, false));
         }
-        CK(cudaMemsetAsync(acc_ovl, 0, (size_t)h->stride * nc * h->limbs * 8, h->fin_stream));
         CK(cudaEventRecord(h->ev_fin[p], h->fin_stream));
         h->fin_pending[p] = true;
         h->par ^= 1;
@@ -574,10 +608,10 @@ int step_phases(st_handle* h, double dt, int phase, bool empty, L&& launch, S&& 
         {
             ProfScope ps(h, ST_KERNEL_FINALIZE);
             CK(launch_finalize(h->limbs, h->dacc, h->dsrc, h->dsrc32, h->dctl, nullptr,
-                               h->dcounter, nc, h->stride, finalize_grid(h), h->stream));
+                               h->dcounter, nc, h->stride, finalize_grid(h), h->stream,
+                               use_pdl(h)));
             h->launches += 1;
         }
-        CK(cudaMemsetAsync(h->dacc, 0, (size_t)h->stride * nc * h->limbs * 8, h->stream));
     }
     h->steps += 1;
     h->steps_since_sort += 1;
@@ -596,8 +630,15 @@ int do_step(st_handle* h, double dt, double fscale, int phase = PH_ALL)
         if (h->tet) return do_step_tet<V>(h, dt, fscale, phase);
     }
     if (!h->capturing && h->clouds_dirty && (rc = upload_clouds<P, V>(h)) != ST_OK) return rc;
-    const bool ovl = h->fin_overlap && phase == PH_ALL && !h->capturing &&
-                     (h->dep == DEP_DET1 || h->dep == DEP_DET2) && h->p.n_clouds == 1;
+    /* Where the overlapped finalize pays: always against a finalize that waits for a plain
+     * launch behind the step (1e4 parcels on 20^3 cells 11.6 against 13.0 us per step, 1e6 on
+     * 64^3 32.0 against 33.9), and against one launched programmatically where the ring runs
+     * (1e7 on 128^3: 230.8 against 234.6 us).  Below that the second stream's events and extra
+     * launches cost more than they hide (9.5 against 10.3 us, 1e5 on 32^3 12.3 against 13.2). */
+    const bool ring = h->p.n_clouds == 1 && use_ring(h, h->clouds[0].n);
+    const bool ovl = h->fin_overlap && h->p.n_clouds == 1 && (ring || !use_pdl(h)) &&
+                     phase == PH_ALL && !h->capturing &&
+                     (h->dep == DEP_DET1 || h->dep == DEP_DET2);
     if ((rc = ovl ? ensure_overlap(h) : join_fin(h))) return rc;
     StepArgs<P, V> a;
     a.mesh = mesh_k<P>(h);
@@ -636,9 +677,9 @@ int do_step(st_handle* h, double dt, double fscale, int phase = PH_ALL)
     if (grid > need) grid = (int)need;
     if (grid < 1) grid = 1;
     auto launch = [&](int dep) -> cudaError_t {
-        if (dep != DEP_PROBE && h->ring && ring_eligible<P, V>(a, dep))
-            return launch_step_ring<P, V>(a, dep, h->nsm, h->stream);
-        return launch_step<P, V>(a, dep, grid, h->block, h->stream);
+        if (dep != DEP_PROBE && ring && ring_eligible<P, V>(a, dep))
+            return launch_step_ring<P, V>(a, dep, h->nsm, h->stream, use_pdl(h));
+        return launch_step<P, V>(a, dep, grid, h->block, h->stream, use_pdl(h));
     };
     return step_phases(h, dt, phase, a.total_tiles == 0, launch,
                        [&] { return do_sort_all<P, V>(h); }, acc_ovl);
@@ -679,9 +720,9 @@ int do_step_tet(st_handle* h, double dt, double fscale, int phase)
     if (grid > need) grid = (int)need;
     if (grid < 1) grid = 1;
     auto launch = [&](int dep) -> cudaError_t {
-        if (dep != DEP_PROBE && h->ring && tet_ring_eligible<V>(a, dep))
-            return launch_step_tet_ring<V>(a, dep, h->nsm, h->stream);
-        return launch_step_tet<V>(a, dep, grid, h->block, h->stream);
+        if (dep != DEP_PROBE && use_ring(h, a.one.n) && tet_ring_eligible<V>(a, dep))
+            return launch_step_tet_ring<V>(a, dep, h->nsm, h->stream, use_pdl(h));
+        return launch_step_tet<V>(a, dep, grid, h->block, h->stream, use_pdl(h));
     };
     return step_phases(h, dt, phase, a.total_tiles == 0, launch,
                        [&] { return do_sort_all<double, V>(h); });
@@ -2128,7 +2169,7 @@ int st_set_step_kernel(st_handle* h, int kind)
     if ((rc = check_handle(h))) return rc;
     if (kind != ST_STEP_KERNEL_RING && kind != ST_STEP_KERNEL_WARP)
         return fail(ST_ERR_INVALID_ARGUMENT, "st_set_step_kernel: unknown kind %d", kind);
-    h->ring = (kind == ST_STEP_KERNEL_RING);
+    h->kernel = kind;
     return ST_OK;
 }
 

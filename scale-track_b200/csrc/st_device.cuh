@@ -18,6 +18,18 @@ namespace st {
 #define FULL_MASK 0xffffffffu
 #endif
 
+/* Programmatic dependent launch: waits until the kernel before this one on the stream has
+ * finished and its writes are visible (at once in a plain launch), and lets the kernel after
+ * this one be set up while this one runs. */
+__device__ __forceinline__ void grid_dep_wait()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dep_launch()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ float st_sqrt(float v) { return __fsqrt_rn(v); }
 __device__ __forceinline__ double st_sqrt(double v) { return __dsqrt_rn(v); }
 

@@ -147,7 +147,7 @@ struct TetStepArgs {
 
 template <class V>
 cudaError_t launch_step_tet(const TetStepArgs<V>& a, int dep, int grid, int block,
-                            cudaStream_t s);
+                            cudaStream_t s, bool pdl = false);
 template <class V>
 int step_tet_max_active_blocks(int dep, int block);
 /* The tet step of a single cloud as a shared-memory ring (st_ring.cuh): true when it can run
@@ -155,7 +155,8 @@ int step_tet_max_active_blocks(int dep, int block);
 template <class V>
 bool tet_ring_eligible(const TetStepArgs<V>& a, int dep);
 template <class V>
-cudaError_t launch_step_tet_ring(const TetStepArgs<V>& a, int dep, int nsm, cudaStream_t s);
+cudaError_t launch_step_tet_ring(const TetStepArgs<V>& a, int dep, int nsm, cudaStream_t s,
+                                 bool pdl = false);
 template <class V>
 cudaError_t tet_ring_prepare();
 /* Walks every parcel from hint[i] to the tet that contains it (hop limit of the mesh);
@@ -212,15 +213,37 @@ cudaError_t launch_adj_mean(const unsigned long long* acc, const CloudCtl* ctl, 
 /* Sets the thread-local message returned by st_last_error (st_abi.cu). */
 void st_set_last_error(const char* msg);
 
+/* Launches a kernel whose launch and block set-up may overlap the end of the kernel before it
+ * on the stream (programmatic dependent launch, pdl = true).  The kernel calls
+ * grid_dep_wait() before it touches memory. */
+template <class... K, class... A>
+cudaError_t launch_kernel(bool pdl, void (*kernel)(K...), dim3 grid, dim3 block, size_t smem,
+                          cudaStream_t s, const A&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+}
+
 /* Launchers implemented in st_kernels.cu (all asynchronous on `s`). */
 template <class P, class V>
-cudaError_t launch_step(const StepArgs<P, V>& a, int dep, int grid, int block, cudaStream_t s);
+cudaError_t launch_step(const StepArgs<P, V>& a, int dep, int grid, int block, cudaStream_t s,
+                        bool pdl = false);
 template <class P, class V>
 int step_max_active_blocks(int dep, int block);
 /* The step of a single cloud as a persistent shared-memory ring (st_ring.cu); deposits
  * DEP_DET1, DEP_DET2 or DEP_ATOMIC.  Every parcel array must be 16-byte aligned. */
 template <class P, class V>
-cudaError_t launch_step_ring(const StepArgs<P, V>& a, int dep, int nsm, cudaStream_t s);
+cudaError_t launch_step_ring(const StepArgs<P, V>& a, int dep, int nsm, cudaStream_t s,
+                             bool pdl = false);
 /* Shared-memory opt-in of the ring kernels of a precision on the current device. */
 template <class P, class V>
 cudaError_t ring_prepare();
@@ -228,11 +251,12 @@ cudaError_t ring_prepare();
 template <class P, class V>
 bool ring_eligible(const StepArgs<P, V>& a, int dep);
 
+constexpr size_t FINALIZE_CLEAR_BYTES = (size_t)64 << 20;   /* launch_finalize */
 /* Fixed point -> FP64 source [nclouds][stride] (and, when src32 is not null, its FP32
  * rounding in the same layout), next scale per cloud. */
 cudaError_t launch_finalize(int limbs, unsigned long long* acc, double* src, float* src32,
                             CloudCtl* ctl, const int32_t* Lsrc, unsigned int* counter,
-                            int nclouds, int64_t stride, int grid_x, cudaStream_t s);
+                            int nclouds, int64_t stride, int grid_x, cudaStream_t s, bool pdl);
 /* Scale of the step just run -> Lfin, next scale from its largest deposit (overlapped
  * finalize: the finalize then reads Lfin). */
 cudaError_t launch_next_scale(CloudCtl* ctl, int32_t* Lfin, int nclouds, cudaStream_t s);

@@ -54,12 +54,16 @@ __device__ __forceinline__ int find_cloud(const StepArgs<P, V>& a, int64_t tile)
  * reduced.  Tiles are distributed over the persistent grid with a fixed stride; the clouds
  * of a multi-cloud launch occupy consecutive tile ranges. */
 /* Resident blocks of 256 threads per SM the compiler must allow (a register budget):
- * 3 (80 registers), which holds the two tiles of the software pipeline without spills. */
+ * 3 (80 registers), which holds the two tiles of the software pipeline without spills; FP64
+ * velocities with one substep 2 (128 registers; 80 spill: 1e5 parcels 17.2 -> 15.0 us per
+ * step, 4e5 26.6 -> 24.9 us).  Several substeps stay at 3 in every precision (mixed, 4e6
+ * parcels with ten substeps: 2 blocks 373 us, 3 blocks 333 us, 4 blocks 430 us; FP64, 2e6 with
+ * four: 2 blocks 180 us, 3 blocks 164 us). */
 #ifndef ST_MIN_BLOCKS
 #define ST_MIN_BLOCKS 3
 #endif
 #ifndef ST_MIN_BLOCKS_FP64
-#define ST_MIN_BLOCKS_FP64 3
+#define ST_MIN_BLOCKS_FP64 2
 #endif
 /* Several substeps per call (the multi-cloud workload) keep more state live per parcel. */
 #ifndef ST_MIN_BLOCKS_SUB
@@ -68,7 +72,7 @@ __device__ __forceinline__ int find_cloud(const StepArgs<P, V>& a, int64_t tile)
 template <class V, bool ONE>
 struct MinBlocks {
     static constexpr int value =
-        sizeof(V) == 8 ? ST_MIN_BLOCKS_FP64 : (ONE ? ST_MIN_BLOCKS : ST_MIN_BLOCKS_SUB);
+        ONE ? (sizeof(V) == 8 ? ST_MIN_BLOCKS_FP64 : ST_MIN_BLOCKS) : ST_MIN_BLOCKS_SUB;
 };
 
 template <class P, class V, int DEP, bool ONE, bool SINGLE>
@@ -81,10 +85,12 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
 
     __shared__ unsigned long long dep_ws[8][dep_ws_words<DEP, V>];
     unsigned long long* const ws = dep_ws[threadIdx.x >> 5];
+    grid_dep_launch();
     if (!ONE) {   /* the table of x^0.687 serves the multi-substep loop */
         pow_tab_fill();
         __syncthreads();
     }
+    grid_dep_wait();
     int cur = -1;
     Quant qp = {0.0, 0.0, 0};
     AmaxT<V> amax = (V)0;
@@ -206,25 +212,25 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
 
 template <class P, class V, bool ONE, bool SINGLE>
 static cudaError_t launch_step_t(const StepArgs<P, V>& a, int dep, int grid, int block,
-                                 cudaStream_t s)
+                                 cudaStream_t s, bool pdl)
 {
     switch (dep) {
-    case det_mode<V>: k_step<P, V, det_mode<V>, ONE, SINGLE><<<grid, block, 0, s>>>(a); break;
-    case DEP_ATOMIC: k_step<P, V, DEP_ATOMIC, ONE, SINGLE><<<grid, block, 0, s>>>(a); break;
-    case DEP_PROBE: k_step<P, V, DEP_PROBE, ONE, SINGLE><<<grid, block, 0, s>>>(a); break;
+    case det_mode<V>: return launch_kernel(pdl, k_step<P, V, det_mode<V>, ONE, SINGLE>, grid, block, 0, s, a);
+    case DEP_ATOMIC: return launch_kernel(pdl, k_step<P, V, DEP_ATOMIC, ONE, SINGLE>, grid, block, 0, s, a);
+    case DEP_PROBE: return launch_kernel(pdl, k_step<P, V, DEP_PROBE, ONE, SINGLE>, grid, block, 0, s, a);
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 template <class P, class V>
-cudaError_t launch_step(const StepArgs<P, V>& a, int dep, int grid, int block, cudaStream_t s)
+cudaError_t launch_step(const StepArgs<P, V>& a, int dep, int grid, int block, cudaStream_t s,
+                        bool pdl)
 {
     if (a.nclouds == 1)
-        return a.phys.nsub == 1 ? launch_step_t<P, V, true, true>(a, dep, grid, block, s)
-                                : launch_step_t<P, V, false, true>(a, dep, grid, block, s);
-    return a.phys.nsub == 1 ? launch_step_t<P, V, true, false>(a, dep, grid, block, s)
-                            : launch_step_t<P, V, false, false>(a, dep, grid, block, s);
+        return a.phys.nsub == 1 ? launch_step_t<P, V, true, true>(a, dep, grid, block, s, pdl)
+                                : launch_step_t<P, V, false, true>(a, dep, grid, block, s, pdl);
+    return a.phys.nsub == 1 ? launch_step_t<P, V, true, false>(a, dep, grid, block, s, pdl)
+                            : launch_step_t<P, V, false, false>(a, dep, grid, block, s, pdl);
 }
 
 template <class P, class V, bool ONE, bool SINGLE>
@@ -253,9 +259,12 @@ int step_max_active_blocks(int dep, int block)
     return m;
 }
 
-template cudaError_t launch_step<float, float>(const StepArgs<float, float>&, int, int, int, cudaStream_t);
-template cudaError_t launch_step<double, float>(const StepArgs<double, float>&, int, int, int, cudaStream_t);
-template cudaError_t launch_step<double, double>(const StepArgs<double, double>&, int, int, int, cudaStream_t);
+template cudaError_t launch_step<float, float>(const StepArgs<float, float>&, int, int, int, cudaStream_t,
+                                                  bool);
+template cudaError_t launch_step<double, float>(const StepArgs<double, float>&, int, int, int, cudaStream_t,
+                                                  bool);
+template cudaError_t launch_step<double, double>(const StepArgs<double, double>&, int, int, int, cudaStream_t,
+                                                  bool);
 template int step_max_active_blocks<float, float>(int, int);
 template int step_max_active_blocks<double, float>(int, int);
 template int step_max_active_blocks<double, double>(int, int);
@@ -264,7 +273,35 @@ template int step_max_active_blocks<double, double>(int, int);
 /* source finalize: fixed point -> FP64, clear accumulators, next scale                 */
 /* ------------------------------------------------------------------------------------ */
 
-template <int LIMBS>
+/* 32-byte accesses (one 32-byte sector per thread): two 16-byte accesses at a 32-byte stride
+ * would touch every sector twice. */
+__device__ __forceinline__ void ld32(const unsigned long long* p, unsigned long long v[4])
+{
+    asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
+                 : "l"(__cvta_generic_to_global(p)));
+}
+__device__ __forceinline__ void ld32_stream(const unsigned long long* p, unsigned long long v[4])
+{
+    asm volatile("ld.global.cs.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
+                 : "l"(__cvta_generic_to_global(p)));
+}
+__device__ __forceinline__ void st32(unsigned long long* p, unsigned long long v)
+{
+    asm volatile("st.global.v4.u64 [%0], {%1, %1, %1, %1};" ::"l"(__cvta_generic_to_global(p)),
+                 "l"(v)
+                 : "memory");
+}
+__device__ __forceinline__ void st32_stream(double* p, const double v[4])
+{
+    asm volatile("st.global.cs.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(
+                     __cvta_generic_to_global(p)),
+                 "d"(v[0]), "d"(v[1]), "d"(v[2]), "d"(v[3])
+                 : "memory");
+}
+
+template <int LIMBS, bool CLEAR>
 __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict__ acc,
                                                   double* __restrict__ src,
                                                   float* __restrict__ src32, CloudCtl* ctl,
@@ -272,44 +309,49 @@ __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict
                                                   unsigned int* counter, int nclouds,
                                                   int64_t stride)
 {
-    /* stride: per-cloud component count, a multiple of 4 (padding stays zero).  The caller
-     * clears the accumulators after this kernel.  Lsrc: the scale of each cloud when the next
-     * scale was already set by k_next_scale (overlapped finalize), else null. */
+    /* stride: per-cloud component count, a multiple of 4 (padding stays zero).  Lsrc: the
+     * scale of each cloud when the next scale was already set by k_next_scale (overlapped
+     * finalize), else null. */
+    grid_dep_launch();
+    grid_dep_wait();
     const int c = blockIdx.y;
     const int L = Lsrc ? Lsrc[c] : ctl[c].L;
-    const ulonglong2* a = reinterpret_cast<const ulonglong2*>(acc + (int64_t)c * stride * LIMBS);
-    double2* s = reinterpret_cast<double2*>(src + (int64_t)c * stride);
-    float4* s32 = src32 ? reinterpret_cast<float4*>(src32 + (int64_t)c * stride) : nullptr;
+    unsigned long long* const a = acc + (int64_t)c * stride * LIMBS;
+    double* const s = src + (int64_t)c * stride;
+    float4* const s32 = src32 ? reinterpret_cast<float4*>(src32 + (int64_t)c * stride) : nullptr;
     const int64_t ngroups = stride / 4;
     const int64_t gstride = (int64_t)gridDim.x * blockDim.x;
-    /* read-only pass: the accumulators are cleared afterwards by a memset, which costs less
-     * than writing zeros back into the lines just read; the source is streamed out */
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += gstride) {
-        double v[4];
-        if (LIMBS == 1) {
-            ulonglong2 q0 = __ldcs(a + 2 * g);
-            ulonglong2 q1 = __ldcs(a + 2 * g + 1);
-            v[0] = (double)(long long)q0.x;
-            v[1] = (double)(long long)q0.y;
-            v[2] = (double)(long long)q1.x;
-            v[3] = (double)(long long)q1.y;
-        } else {
-            ulonglong2 q[4];
+        unsigned long long q[4 * LIMBS];
+        unsigned long long any = 0;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) q[k] = __ldcs(a + 4 * g + k);
+        for (int l = 0; l < LIMBS; ++l) {
+            if (CLEAR) ld32(a + 4 * (LIMBS * g + l), q + 4 * l);
+            else ld32_stream(a + 4 * (LIMBS * g + l), q + 4 * l);
+        }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                long long hi = (long long)q[k].x;
-                unsigned long long lo = q[k].y;
+        for (int k = 0; k < 4 * LIMBS; ++k) any |= q[k];
+        double o[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            double v;
+            if (LIMBS == 1) {
+                v = (double)(long long)q[k];
+            } else {
+                long long hi = (long long)q[2 * k];
+                unsigned long long lo = q[2 * k + 1];
                 hi += (long long)(lo >> 32);
                 lo &= 0xffffffffULL;
-                v[k] = (double)hi * 4294967296.0 + (double)lo;
+                v = (double)hi * 4294967296.0 + (double)lo;
             }
+            o[k] = ldexp2(v, L);
         }
-        const double o[4] = {ldexp2(v[0], L), ldexp2(v[1], L), ldexp2(v[2], L),
-                             ldexp2(v[3], L)};
-        __stcs(s + 2 * g, make_double2(o[0], o[1]));
-        __stcs(s + 2 * g + 1, make_double2(o[2], o[3]));
+        st32_stream(s + 4 * g, o);
+        /* cleared for the step after, where there is anything to clear */
+        if (CLEAR && any) {
+#pragma unroll
+            for (int l = 0; l < LIMBS; ++l) st32(a + 4 * (LIMBS * g + l), 0ULL);
+        }
         /* a 4-byte copy for an FP32 exchange array, rounded once from the FP64 source */
         if (s32) __stcs(s32 + g, make_float4((float)o[0], (float)o[1], (float)o[2], (float)o[3]));
     }
@@ -333,17 +375,25 @@ __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict
     }
 }
 
+/* Accumulators up to FINALIZE_CLEAR_BYTES are cleared by the conversion as it reads them, which saves the
+ * memset's launch behind every step (1e4 parcels on 20^3 cells: 16.2 -> 13.0 us per step, 4e6
+ * on 64^3: 92.8 -> 88.6 us); 128^3 cells (50 MB) are even.  Larger ones exceed the L2 together
+ * with the source and U: there zeros written between the reads are slower than a memset of
+ * its own (64 sources of 64^3 cells, 403 MB: 1462 against 1358 us per step). */
 cudaError_t launch_finalize(int limbs, unsigned long long* acc, double* src, float* src32,
                             CloudCtl* ctl, const int32_t* Lsrc, unsigned int* counter,
-                            int nclouds, int64_t stride, int grid_x, cudaStream_t s)
+                            int nclouds, int64_t stride, int grid_x, cudaStream_t s, bool pdl)
 {
     if (stride % 4) return cudaErrorInvalidValue;
     dim3 grid(grid_x, nclouds);
-    if (limbs == 1)
-        k_finalize<1><<<grid, 256, 0, s>>>(acc, src, src32, ctl, Lsrc, counter, nclouds, stride);
-    else
-        k_finalize<2><<<grid, 256, 0, s>>>(acc, src, src32, ctl, Lsrc, counter, nclouds, stride);
-    return cudaGetLastError();
+    const size_t bytes = (size_t)stride * nclouds * limbs * 8;
+    const bool clear = bytes <= FINALIZE_CLEAR_BYTES;
+    const auto k = limbs == 1 ? (clear ? k_finalize<1, true> : k_finalize<1, false>)
+                              : (clear ? k_finalize<2, true> : k_finalize<2, false>);
+    const cudaError_t e = launch_kernel(pdl, k, grid, dim3(256), 0, s, acc, src, src32, ctl, Lsrc,
+                                        counter, nclouds, stride);
+    if (e != cudaSuccess || clear) return e;
+    return cudaMemsetAsync(acc, 0, bytes, s);
 }
 
 /* The scale bookkeeping of k_finalize on its own, for an overlapped finalize: keeps each

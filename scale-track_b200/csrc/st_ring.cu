@@ -142,6 +142,8 @@ __global__ void __launch_bounds__(HexShapeOf<V>::type::THREADS, 1)
 {
     using HexShape = typename HexShapeOf<V>::type;
     constexpr bool DET = (DEP == DEP_DET1 || DEP == DEP_DET2);
+    grid_dep_launch();
+    grid_dep_wait();
     Quant qp = {0.0, 0.0, 0.0f, 0.0f, 0, false};
     if (DET) qp = make_quant(a.ctl[0].L, a.ctl[0].H + QUANT_GROWTH_BITS);
     AmaxT<V> amax = (V)0;
@@ -181,7 +183,7 @@ static cudaError_t ring_attr()
 }
 
 template <class P, class V, int DEP, bool ONE>
-static cudaError_t launch_ring_t(const StepArgs<P, V>& a, int nsm, cudaStream_t s)
+static cudaError_t launch_ring_t(const StepArgs<P, V>& a, int nsm, cudaStream_t s, bool pdl)
 {
     using HexShape = typename HexShapeOf<V>::type;
     cudaError_t e = ring_attr<P, V, DEP, ONE>();
@@ -189,9 +191,8 @@ static cudaError_t launch_ring_t(const StepArgs<P, V>& a, int nsm, cudaStream_t 
     const int64_t nfull = a.one.n / HexShape::BT;
     int64_t grid = nfull < nsm ? nfull : nsm;
     if (grid < 1) grid = 1;
-    k_step_ring<P, V, DEP, ONE>
-        <<<(int)grid, HexShape::THREADS, RingGeom<HexShape, P, V, false>::SMEM, s>>>(a);
-    return cudaGetLastError();
+    return launch_kernel(pdl, k_step_ring<P, V, DEP, ONE>, (int)grid, HexShape::THREADS,
+                         RingGeom<HexShape, P, V, false>::SMEM, s, a);
 }
 
 /* Makes every ring kernel instance of a precision launchable on the current device (called
@@ -220,22 +221,22 @@ bool ring_eligible(const StepArgs<P, V>& a, int dep)
 }
 
 template <class P, class V>
-cudaError_t launch_step_ring(const StepArgs<P, V>& a, int dep, int nsm, cudaStream_t s)
+cudaError_t launch_step_ring(const StepArgs<P, V>& a, int dep, int nsm, cudaStream_t s, bool pdl)
 {
     if (a.nclouds != 1) return cudaErrorInvalidValue;
     const bool one = a.phys.nsub == 1;
     switch (dep) {
-    case det_mode<V>: return one ? launch_ring_t<P, V, det_mode<V>, true>(a, nsm, s)
-                                 : launch_ring_t<P, V, det_mode<V>, false>(a, nsm, s);
-    case DEP_ATOMIC: return one ? launch_ring_t<P, V, DEP_ATOMIC, true>(a, nsm, s)
-                                : launch_ring_t<P, V, DEP_ATOMIC, false>(a, nsm, s);
+    case det_mode<V>: return one ? launch_ring_t<P, V, det_mode<V>, true>(a, nsm, s, pdl)
+                                 : launch_ring_t<P, V, det_mode<V>, false>(a, nsm, s, pdl);
+    case DEP_ATOMIC: return one ? launch_ring_t<P, V, DEP_ATOMIC, true>(a, nsm, s, pdl)
+                                : launch_ring_t<P, V, DEP_ATOMIC, false>(a, nsm, s, pdl);
     default: return cudaErrorInvalidValue;
     }
 }
 
-template cudaError_t launch_step_ring<float, float>(const StepArgs<float, float>&, int, int, cudaStream_t);
-template cudaError_t launch_step_ring<double, float>(const StepArgs<double, float>&, int, int, cudaStream_t);
-template cudaError_t launch_step_ring<double, double>(const StepArgs<double, double>&, int, int, cudaStream_t);
+template cudaError_t launch_step_ring<float, float>(const StepArgs<float, float>&, int, int, cudaStream_t, bool);
+template cudaError_t launch_step_ring<double, float>(const StepArgs<double, float>&, int, int, cudaStream_t, bool);
+template cudaError_t launch_step_ring<double, double>(const StepArgs<double, double>&, int, int, cudaStream_t, bool);
 template cudaError_t ring_prepare<float, float>();
 template cudaError_t ring_prepare<double, float>();
 template cudaError_t ring_prepare<double, double>();

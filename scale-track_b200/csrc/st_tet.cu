@@ -303,13 +303,18 @@ __device__ __forceinline__ void tet_parcel(const TetStepArgs<V>& a, int nsub, do
     cell = tNew;
 }
 
-/* Resident blocks of 256 threads per SM the compiler must allow: 4 (64 registers). */
+/* Resident blocks of 256 threads per SM the compiler must allow: 4 (64 registers); FP64
+ * velocities 3 (80 registers), which ends most of their spills (5e4 parcels with two substeps:
+ * 23.2 -> 21.4 us per step, 1e6 parcels with one: 67.9 -> 64.6 us). */
 #ifndef ST_TET_MIN_BLOCKS
 #define ST_TET_MIN_BLOCKS 4
 #endif
+#ifndef ST_TET_MIN_BLOCKS_FP64
+#define ST_TET_MIN_BLOCKS_FP64 3
+#endif
 template <class V>
 struct TetMinBlocks {
-    static constexpr int value = ST_TET_MIN_BLOCKS;
+    static constexpr int value = sizeof(V) == 8 ? ST_TET_MIN_BLOCKS_FP64 : ST_TET_MIN_BLOCKS;
 };
 
 template <class V, int DEP, bool ONE>
@@ -328,6 +333,8 @@ __global__ void __launch_bounds__(256, TetMinBlocks<V>::value) k_step_tet(const 
     const bool count_hops = a.hop_hist != nullptr && DEP != DEP_PROBE;
     __shared__ unsigned long long dep_ws[8][dep_ws_words<DEP, V>];
     unsigned long long* const ws = dep_ws[threadIdx.x >> 5];
+    grid_dep_launch();
+    grid_dep_wait();
     if (threadIdx.x < 8) s_tet_hist[threadIdx.x] = 0;
     __syncthreads();
 
@@ -442,6 +449,8 @@ template <class V, int DEP, bool ONE>
 __global__ void __launch_bounds__(TetShape::THREADS, 1) k_step_tet_ring(const TetStepArgs<V> a)
 {
     constexpr bool DET = (DEP == DEP_DET1 || DEP == DEP_DET2);
+    grid_dep_launch();
+    grid_dep_wait();
     Quant qp = {0.0, 0.0, 0.0f, 0.0f, 0, false};
     if (DET) qp = make_quant(a.ctl[0].L, a.ctl[0].H + QUANT_GROWTH_BITS);
     AmaxT<V> amax = (V)0;
@@ -482,16 +491,15 @@ static cudaError_t tet_ring_attr()
 }
 
 template <class V, int DEP, bool ONE>
-static cudaError_t launch_tet_ring_t(const TetStepArgs<V>& a, int nsm, cudaStream_t s)
+static cudaError_t launch_tet_ring_t(const TetStepArgs<V>& a, int nsm, cudaStream_t s, bool pdl)
 {
     cudaError_t e = tet_ring_attr<V, DEP, ONE>();
     if (e != cudaSuccess) return e;
     const int64_t nfull = a.one.n / TetShape::BT;
     int64_t grid = nfull < nsm ? nfull : nsm;
     if (grid < 1) grid = 1;
-    k_step_tet_ring<V, DEP, ONE>
-        <<<(int)grid, TetShape::THREADS, RingGeom<TetShape, double, V, true>::SMEM, s>>>(a);
-    return cudaGetLastError();
+    return launch_kernel(pdl, k_step_tet_ring<V, DEP, ONE>, (int)grid, TetShape::THREADS,
+                         RingGeom<TetShape, double, V, true>::SMEM, s, a);
 }
 
 template <class V>
@@ -506,14 +514,15 @@ bool tet_ring_eligible(const TetStepArgs<V>& a, int dep)
 }
 
 template <class V>
-cudaError_t launch_step_tet_ring(const TetStepArgs<V>& a, int dep, int nsm, cudaStream_t s)
+cudaError_t launch_step_tet_ring(const TetStepArgs<V>& a, int dep, int nsm, cudaStream_t s,
+                                 bool pdl)
 {
     const bool one = a.phys.nsub == 1;
     switch (dep) {
-    case det_mode<V>: return one ? launch_tet_ring_t<V, det_mode<V>, true>(a, nsm, s)
-                                 : launch_tet_ring_t<V, det_mode<V>, false>(a, nsm, s);
-    case DEP_ATOMIC: return one ? launch_tet_ring_t<V, DEP_ATOMIC, true>(a, nsm, s)
-                                : launch_tet_ring_t<V, DEP_ATOMIC, false>(a, nsm, s);
+    case det_mode<V>: return one ? launch_tet_ring_t<V, det_mode<V>, true>(a, nsm, s, pdl)
+                                 : launch_tet_ring_t<V, det_mode<V>, false>(a, nsm, s, pdl);
+    case DEP_ATOMIC: return one ? launch_tet_ring_t<V, DEP_ATOMIC, true>(a, nsm, s, pdl)
+                                : launch_tet_ring_t<V, DEP_ATOMIC, false>(a, nsm, s, pdl);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -534,29 +543,29 @@ cudaError_t tet_ring_prepare()
 
 template bool tet_ring_eligible<float>(const TetStepArgs<float>&, int);
 template bool tet_ring_eligible<double>(const TetStepArgs<double>&, int);
-template cudaError_t launch_step_tet_ring<float>(const TetStepArgs<float>&, int, int, cudaStream_t);
-template cudaError_t launch_step_tet_ring<double>(const TetStepArgs<double>&, int, int, cudaStream_t);
+template cudaError_t launch_step_tet_ring<float>(const TetStepArgs<float>&, int, int, cudaStream_t, bool);
+template cudaError_t launch_step_tet_ring<double>(const TetStepArgs<double>&, int, int, cudaStream_t, bool);
 template cudaError_t tet_ring_prepare<float>();
 template cudaError_t tet_ring_prepare<double>();
 
 template <class V, bool ONE>
 static cudaError_t launch_step_tet_t(const TetStepArgs<V>& a, int dep, int grid, int block,
-                                     cudaStream_t s)
+                                     cudaStream_t s, bool pdl)
 {
     switch (dep) {
-    case det_mode<V>: k_step_tet<V, det_mode<V>, ONE><<<grid, block, 0, s>>>(a); break;
-    case DEP_ATOMIC: k_step_tet<V, DEP_ATOMIC, ONE><<<grid, block, 0, s>>>(a); break;
-    case DEP_PROBE: k_step_tet<V, DEP_PROBE, ONE><<<grid, block, 0, s>>>(a); break;
+    case det_mode<V>: return launch_kernel(pdl, k_step_tet<V, det_mode<V>, ONE>, grid, block, 0, s, a);
+    case DEP_ATOMIC: return launch_kernel(pdl, k_step_tet<V, DEP_ATOMIC, ONE>, grid, block, 0, s, a);
+    case DEP_PROBE: return launch_kernel(pdl, k_step_tet<V, DEP_PROBE, ONE>, grid, block, 0, s, a);
     default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
 }
 
 template <class V>
-cudaError_t launch_step_tet(const TetStepArgs<V>& a, int dep, int grid, int block, cudaStream_t s)
+cudaError_t launch_step_tet(const TetStepArgs<V>& a, int dep, int grid, int block, cudaStream_t s,
+                            bool pdl)
 {
-    return a.phys.nsub == 1 ? launch_step_tet_t<V, true>(a, dep, grid, block, s)
-                            : launch_step_tet_t<V, false>(a, dep, grid, block, s);
+    return a.phys.nsub == 1 ? launch_step_tet_t<V, true>(a, dep, grid, block, s, pdl)
+                            : launch_step_tet_t<V, false>(a, dep, grid, block, s, pdl);
 }
 
 template <class V, bool ONE>
@@ -610,8 +619,8 @@ cudaError_t launch_tet_locate(const TetMeshK& m, const double* x, const double* 
     return cudaGetLastError();
 }
 
-template cudaError_t launch_step_tet<float>(const TetStepArgs<float>&, int, int, int, cudaStream_t);
-template cudaError_t launch_step_tet<double>(const TetStepArgs<double>&, int, int, int, cudaStream_t);
+template cudaError_t launch_step_tet<float>(const TetStepArgs<float>&, int, int, int, cudaStream_t, bool);
+template cudaError_t launch_step_tet<double>(const TetStepArgs<double>&, int, int, int, cudaStream_t, bool);
 template int step_tet_max_active_blocks<float>(int, int);
 template int step_tet_max_active_blocks<double>(int, int);
 
