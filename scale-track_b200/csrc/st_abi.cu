@@ -102,11 +102,10 @@ struct AdjTape {
     void* mem = nullptr;        /* one allocation, carved below */
     void* ck_x = nullptr;
     void* ck_v = nullptr;
-    void* rec_v = nullptr;
-    int32_t* rec_c = nullptr;
-    uint8_t* rec_b = nullptr;
-    double* G = nullptr;
-    void* adj_v = nullptr;
+    unsigned char* rec = nullptr;
+    double* ybar = nullptr;
+    void* G = nullptr;
+    double* dv0 = nullptr;
     double* partials = nullptr;
     void* fsd = nullptr;
     double* mean = nullptr;
@@ -1228,18 +1227,17 @@ int adj_prepare(st_handle* h, int cloud, const st_adjoint_desc* d)
     const int64_t n = h->clouds[cloud].n;
     const int T = d->n_steps, C = d->checkpoint_interval;
     const int nseg = (T + C - 1) / C;
-    const int grid = (int)((n + 255) / 256);
+    const int grid = adj_reverse_grid<P, V>(n, h->nsm);
     const int limbs = sizeof(V) == 8 ? 2 : 1;
     size_t off = 0;
     auto carve = [&](size_t b) { size_t o = off; off += align256(b); return o; };
     const size_t o_ckx = carve((size_t)nseg * 3 * n * sizeof(P));
     const size_t o_ckv = carve((size_t)nseg * 3 * n * sizeof(V));
-    const size_t o_rv = carve((size_t)C * 3 * n * sizeof(V));
-    const size_t o_rc = carve((size_t)C * n * sizeof(int32_t));
-    const size_t o_rb = carve((size_t)C * n);
-    const size_t o_G = carve((size_t)h->stride * sizeof(double));
-    const size_t o_av = carve((size_t)3 * n * sizeof(V));
-    const size_t o_pa = carve((size_t)nseg * (grid > 0 ? grid : 1) * 2 * sizeof(double));
+    const size_t o_rec = carve((size_t)grid * C * 256 * adj_rec_bytes<V>);
+    const size_t o_y = carve((size_t)h->stride * sizeof(double));
+    const size_t o_G = carve((size_t)h->stride * sizeof(V));
+    const size_t o_dv = carve((size_t)3 * n * sizeof(double));
+    const size_t o_pa = carve((size_t)((n + 255) / 256 + 1) * 2 * sizeof(double));
     const size_t o_fs = carve((size_t)2 * T * sizeof(V));   /* fs, then fs_lo */
     const size_t o_mean = carve((size_t)h->stride * sizeof(double));
     const size_t o_ctl = carve(sizeof(CloudCtl));
@@ -1252,11 +1250,11 @@ int adj_prepare(st_handle* h, int cloud, const st_adjoint_desc* d)
         t.bytes = off;
     }
     char* b = static_cast<char*>(t.mem);
-    t.ck_x = b + o_ckx; t.ck_v = b + o_ckv; t.rec_v = b + o_rv;
-    t.rec_c = reinterpret_cast<int32_t*>(b + o_rc);
-    t.rec_b = reinterpret_cast<uint8_t*>(b + o_rb);
-    t.G = reinterpret_cast<double*>(b + o_G);
-    t.adj_v = b + o_av;
+    t.ck_x = b + o_ckx; t.ck_v = b + o_ckv;
+    t.rec = reinterpret_cast<unsigned char*>(b + o_rec);
+    t.ybar = reinterpret_cast<double*>(b + o_y);
+    t.G = b + o_G;
+    t.dv0 = reinterpret_cast<double*>(b + o_dv);
     t.partials = reinterpret_cast<double*>(b + o_pa);
     t.fsd = b + o_fs;
     t.mean = reinterpret_cast<double*>(b + o_mean);
@@ -1294,8 +1292,11 @@ AdjArgs<P, V> adj_args(st_handle* h)
     a.fs_lo = (const V*)t.fsd + t.T;
     a.acc = t.acc; a.ctl = t.ctl;
     a.ck_x = (P*)t.ck_x; a.ck_v = (V*)t.ck_v;
-    a.rec_v = (V*)t.rec_v; a.rec_c = t.rec_c; a.rec_b = t.rec_b;
-    a.G = t.G; a.adj_v = (V*)t.adj_v; a.partials = t.partials;
+    a.rec = t.rec;
+    a.G = (const V*)t.G;
+    a.id = c.id[c.cur];
+    a.dv0 = t.dv0;
+    a.partials = t.partials;
     return a;
 }
 
@@ -1350,45 +1351,30 @@ int adj_pullback(st_handle* h, int cloud, const st_adjoint_desc* d, const double
                     "st_mean_source_pullback needs a preceding st_mean_source_forward with the "
                     "same cloud and descriptor");
     const int64_t ncomp = h->ncells * 3;
-    std::vector<double> G(ncomp);
-    for (int64_t j = 0; j < ncomp; ++j) G[j] = cot[j] / (double)t.T;
-    CK(cudaMemcpyAsync(t.G, G.data(), ncomp * sizeof(double), cudaMemcpyHostToDevice,
-                       h->stream));
-    CK(cudaMemsetAsync(t.adj_v, 0, (size_t)3 * t.n * sizeof(V), h->stream));
+    CK(cudaMemcpyAsync(t.ybar, cot, ncomp * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     AdjArgs<P, V> a = adj_args<P, V>(h);
+    if (!dv0) a.dv0 = nullptr;
     {
         ProfScope ps(h, ST_KERNEL_ADJ_REVERSE);
-        for (int seg = t.nseg - 1; seg >= 0; --seg) {
-            const int len = std::min(t.C, t.T - seg * t.C);
-            CK(launch_adj_reverse<P, V>(a, seg, len, t.grid, h->stream));
-            h->launches += 1;
-        }
+        CK(launch_adj_cotangent<V>(t.ybar, t.T, (V*)t.G, ncomp, h->stream));
+        CK(launch_adj_reverse<P, V>(a, t.grid, h->stream));
+        h->launches += t.grid > 0 ? 2 : 1;
     }
-    std::vector<double> parts((size_t)t.nseg * t.grid * 2);
+    std::vector<double> parts((size_t)((t.n + 255) / 256) * 2);
     if (!parts.empty())
         CK(cudaMemcpyAsync(parts.data(), t.partials, parts.size() * sizeof(double),
                            cudaMemcpyDeviceToHost, h->stream));
-    std::vector<V> av(dv0 ? (size_t)3 * t.n : 0);
-    std::vector<int32_t> id(dv0 ? t.n : 0);
-    CloudBufs& c = h->clouds[cloud];
-    if (dv0 && t.n > 0) {
-        CK(cudaMemcpyAsync(av.data(), t.adj_v, av.size() * sizeof(V), cudaMemcpyDeviceToHost,
+    if (dv0 && t.n > 0)
+        CK(cudaMemcpyAsync(dv0, t.dv0, (size_t)3 * t.n * sizeof(double), cudaMemcpyDeviceToHost,
                            h->stream));
-        CK(cudaMemcpyAsync(id.data(), c.id[c.cur], id.size() * sizeof(int32_t),
-                           cudaMemcpyDeviceToHost, h->stream));
-    }
     CK(cudaStreamSynchronize(h->stream));
-    double sa = 0.0, ss = 0.0;  /* fixed order: segment, then block */
+    double sa = 0.0, ss = 0.0;  /* fixed order: 256 parcels after 256 parcels */
     for (size_t k = 0; k < parts.size(); k += 2) {
         sa += parts[k];
         ss += parts[k + 1];
     }
     if (dalpha) *dalpha = sa;
     if (dscale) *dscale = ss;
-    if (dv0)
-        for (int comp = 0; comp < 3; ++comp)
-            for (int64_t j = 0; j < t.n; ++j)
-                dv0[comp * t.n + id[j]] = (double)av[comp * t.n + j];
     return ST_OK;
 }
 

@@ -193,19 +193,25 @@ struct AdjArgs {
     CloudCtl* ctl;              /* scale and counters of the adjoint run */
     P* ck_x;                    /* checkpoints [nseg][3][n] */
     V* ck_v;
-    V* rec_v;                   /* forward records of one segment [C][3][n] */
-    int32_t* rec_c;             /* [C][n] */
-    uint8_t* rec_b;             /* [C][n] */
-    const double* G;            /* dJ/dS_n per cell component [ncomp] */
-    V* adj_v;                   /* velocity cotangent [3][n] */
-    double* partials;           /* [nseg][grid][2] parameter partials */
+    unsigned char* rec;         /* records of one segment, [reverse grid][C * 256 * rec bytes] */
+    const V* G;                 /* dJ/dS_n per cell component [ncomp] */
+    const int32_t* id;          /* st_set_parcels index of each parcel */
+    double* dv0;                /* velocity cotangent [3][n] by that index, or null */
+    double* partials;           /* parameter partials [ceil(n/256)][2] */
 };
+
+/* Bytes of a reverse record: four V, the cell, the bounce flags. */
+template <class V>
+constexpr int adj_rec_bytes = 4 * sizeof(V) + sizeof(int32_t) + 1;
 
 template <class P, class V>
 cudaError_t launch_adj_forward(const AdjArgs<P, V>& a, bool probe, cudaStream_t s);
 template <class P, class V>
-cudaError_t launch_adj_reverse(const AdjArgs<P, V>& a, int seg, int len, int grid,
-                               cudaStream_t s);
+cudaError_t launch_adj_reverse(const AdjArgs<P, V>& a, int grid, cudaStream_t s);
+template <class P, class V>
+int adj_reverse_grid(int64_t n, int nsm);
+template <class V>
+cudaError_t launch_adj_cotangent(const double* ybar, int T, V* G, int64_t ncomp, cudaStream_t s);
 cudaError_t launch_adj_scale(CloudCtl* ctl, cudaStream_t s);
 cudaError_t launch_adj_mean(const unsigned long long* acc, const CloudCtl* ctl, int limbs,
                             int T, double* mean, int64_t ncomp, cudaStream_t s);
