@@ -34,6 +34,7 @@
 
 #include "scaletrack.h"
 #include "st_internal.h"
+#include "st_xfer.h"
 
 using namespace st;
 
@@ -727,6 +728,34 @@ int do_step_tet(st_handle* h, double dt, double fscale, int phase)
                        [&] { return do_sort_all<double, V>(h); });
 }
 
+/* Parcels pass between the caller's arrays and the cloud in chunks of this many, converted
+ * and ordered on the device through the handle's staging array (59 MB). */
+constexpr int64_t PARCEL_CHUNK = (int64_t)1 << 20;
+
+/* The caller's [3][m], [3][m] and [m] arrays into the current buffers at first .. first+m-1. */
+template <class P, class V>
+int import_parcels(st_handle* h, CloudBufs& c, int64_t first, int64_t m, const double* xyz,
+                   const double* uvw, const double* d)
+{
+    int rc;
+    if ((rc = ensure_stage(h, (size_t)std::min(m, PARCEL_CHUNK) * 7 * sizeof(double)))) return rc;
+    double* const st = static_cast<double*>(h->dstage);
+    SortBufs<P, V> b = sort_bufs<P, V>(h, c);
+    for (int64_t o = 0; o < m; o += PARCEL_CHUNK) {
+        const int64_t k = std::min(PARCEL_CHUNK, m - o);
+        XferSeg seg[7];
+        for (int a = 0; a < 7; ++a) {
+            const double* src = (a < 3 ? xyz + a * m : (a < 6 ? uvw + (a - 3) * m : d)) + o;
+            seg[a] = {const_cast<double*>(src), st + a * k, k * sizeof(double)};
+        }
+        CK(xfer_up(seg, 7, h->device, h->stream));
+        ProfScope ps(h, ST_KERNEL_OTHER);
+        CK(import_chunk<P, V>(b, c.cur, first + o, k, st, h->stream));
+        h->launches += 1;
+    }
+    return ST_OK;
+}
+
 /* Parcels generated on the device instead of uploaded (st_init_parcels). */
 struct InitSpec {
     uint64_t seed;
@@ -775,36 +804,16 @@ int do_set_parcels(st_handle* h, int cloud, int64_t n, const double* xyz, const 
         h->launches += 1;
     }
     if (n > 0 && !gen) {
-        std::vector<P> hp(n);
-        std::vector<V> hv(n);
-        std::vector<int32_t> hid(n);
-        for (int a = 0; a < 3; ++a) {
-            for (int64_t i = 0; i < n; ++i) hp[i] = (P)xyz[a * n + i];
-            void* dst = a == 0 ? c.x[0] : (a == 1 ? c.y[0] : c.z[0]);
-            CK(cudaMemcpyAsync(dst, hp.data(), n * sizeof(P), cudaMemcpyHostToDevice, h->stream));
-            CK(cudaStreamSynchronize(h->stream));   /* hp is reused */
-        }
-        for (int a = 0; a < 4; ++a) {
-            const double* srcp = a < 3 ? uvw + a * n : d;
-            for (int64_t i = 0; i < n; ++i) hv[i] = (V)srcp[i];
-            void* dst = a == 0 ? c.u[0] : (a == 1 ? c.v[0] : (a == 2 ? c.w[0] : c.d[0]));
-            CK(cudaMemcpyAsync(dst, hv.data(), n * sizeof(V), cudaMemcpyHostToDevice, h->stream));
-            CK(cudaStreamSynchronize(h->stream));   /* hv is reused */
-        }
-        for (int64_t i = 0; i < n; ++i) hid[i] = (int32_t)i;
-        /* every upload is ordered on the handle's stream: a plain cudaMemcpy runs on the
-         * legacy stream, which the handle's non-blocking stream does not wait for */
-        CK(cudaMemcpyAsync(c.id[0], hid.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice,
-                           h->stream));
-        CK(cudaStreamSynchronize(h->stream));   /* hid is freed at the end of this block */
+        int rc;
+        if ((rc = import_parcels<P, V>(h, c, 0, n, xyz, uvw, d))) return rc;
     }
     if (n > 0) {
         /* every parcel must start inside the mesh: the reference would index out of bounds */
         CK(cudaMemsetAsync(h->dcount, 0, sizeof(unsigned long long), h->stream));
         if (h->tet) {
             /* walk from the caller's hint to the owning tet */
-            CK(cudaMemcpyAsync(c.cell[1], hint, n * sizeof(int32_t), cudaMemcpyHostToDevice,
-                               h->stream));
+            const XferSeg seg = {const_cast<int32_t*>(hint), c.cell[1], n * sizeof(int32_t)};
+            CK(xfer_up(&seg, 1, h->device, h->stream));
             ProfScope ps(h, ST_KERNEL_OTHER);
             TetMeshK lm = h->tmesh;
             lm.hop_limit = 1 << 20;   /* bounded: a walk that cycles counts as outside */
@@ -906,25 +915,8 @@ int do_append_parcels(st_handle* h, int cloud, int64_t m, const double* xyz, con
         h->clouds_dirty = true;
     }
     const int k = c.cur;
-    std::vector<P> hp(m);
-    std::vector<V> hv(m);
-    std::vector<int32_t> hid(m);
+    if (int rc = import_parcels<P, V>(h, c, n, m, xyz, uvw, d)) return rc;
     P* dstp[3] = {(P*)c.x[k] + n, (P*)c.y[k] + n, (P*)c.z[k] + n};
-    for (int a = 0; a < 3; ++a) {
-        for (int64_t i = 0; i < m; ++i) hp[i] = (P)xyz[a * m + i];
-        CK(cudaMemcpyAsync(dstp[a], hp.data(), m * sizeof(P), cudaMemcpyHostToDevice, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-    }
-    V* dstv[4] = {(V*)c.u[k] + n, (V*)c.v[k] + n, (V*)c.w[k] + n, (V*)c.d[k] + n};
-    for (int a = 0; a < 4; ++a) {
-        const double* srcp = a < 3 ? uvw + a * m : d;
-        for (int64_t i = 0; i < m; ++i) hv[i] = (V)srcp[i];
-        CK(cudaMemcpyAsync(dstv[a], hv.data(), m * sizeof(V), cudaMemcpyHostToDevice, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-    }
-    for (int64_t i = 0; i < m; ++i) hid[i] = (int32_t)(n + i);
-    CK(cudaMemcpyAsync(c.id[k] + n, hid.data(), m * sizeof(int32_t), cudaMemcpyHostToDevice,
-                       h->stream));
     /* the new parcels must lie inside the mesh */
     CK(cudaMemsetAsync(h->dcount, 0, sizeof(unsigned long long), h->stream));
     {
@@ -951,29 +943,31 @@ int do_get_parcels(st_handle* h, int cloud, double* xyz, double* uvw, double* d)
     CloudBufs& c = h->clouds[cloud];
     const int64_t n = c.n;
     if (n == 0) return ST_OK;
+    int rc;
+    if ((rc = ensure_stage(h, (size_t)std::min(n, PARCEL_CHUNK) * 7 * sizeof(double)))) return rc;
+    double* const st = static_cast<double*>(h->dstage);
     SortBufs<P, V> b = sort_bufs<P, V>(h, c);
     {
         ProfScope ps(h, ST_KERNEL_OTHER);
-        CK(unpermute_cloud<P, V>(b, c.cur, n, h->stream));
+        CK(export_order<P, V>(b, c.cur, n, h->stream));
         h->launches += 1;
     }
-    const int o = 1 - c.cur;
-    std::vector<P> hp(n);
-    std::vector<V> hv(n);
-    void* ps_[3] = {c.x[o], c.y[o], c.z[o]};
-    for (int a = 0; a < 3; ++a) {
-        CK(cudaMemcpyAsync(hp.data(), ps_[a], n * sizeof(P), cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-        if (xyz)
-            for (int64_t i = 0; i < n; ++i) xyz[a * n + i] = (double)hp[i];
-    }
-    void* vs_[4] = {c.u[o], c.v[o], c.w[o], c.d[o]};
-    for (int a = 0; a < 4; ++a) {
-        double* dst = a < 3 ? (uvw ? uvw + a * n : nullptr) : d;
-        if (!dst) continue;
-        CK(cudaMemcpyAsync(hv.data(), vs_[a], n * sizeof(V), cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-        for (int64_t i = 0; i < n; ++i) dst[i] = (double)hv[i];
+    for (int64_t o = 0; o < n; o += PARCEL_CHUNK) {
+        const int64_t k = std::min(PARCEL_CHUNK, n - o);
+        {
+            ProfScope ps(h, ST_KERNEL_OTHER);
+            CK(export_chunk<P, V>(b, c.cur, o, k, st, h->stream));
+            h->launches += 1;
+        }
+        XferSeg seg[7];
+        int ns = 0;
+        for (int a = 0; a < 7; ++a) {
+            double* dst = a < 3 ? (xyz ? xyz + a * n + o : nullptr)
+                                : (a < 6 ? (uvw ? uvw + (a - 3) * n + o : nullptr)
+                                         : (d ? d + o : nullptr));
+            if (dst) seg[ns++] = {dst, st + a * k, k * sizeof(double)};
+        }
+        CK(xfer_down(seg, ns, h->device, h->stream));
     }
     return ST_OK;
 }
@@ -995,8 +989,8 @@ int do_get_cells(st_handle* h, int cloud, int32_t* cells)
                           c.id[c.cur], n, mesh_k<P>(h), (int32_t*)c.keys[0], nullptr, h->stream));
         h->launches += 1;
     }
-    CK(cudaMemcpyAsync(cells, c.keys[0], n * sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    const XferSeg seg = {cells, c.keys[0], n * sizeof(int32_t)};
+    CK(xfer_down(&seg, 1, h->device, h->stream));
     return ST_OK;
 }
 
@@ -1326,9 +1320,10 @@ int adj_forward(st_handle* h, int cloud, const st_adjoint_desc* d, double* mean_
     }
     CloudCtl out;
     CK(cudaMemcpyAsync(&out, t.ctl, sizeof out, cudaMemcpyDeviceToHost, h->stream));
-    if (mean_out)
-        CK(cudaMemcpyAsync(mean_out, t.mean, h->ncells * 3 * sizeof(double),
-                           cudaMemcpyDeviceToHost, h->stream));
+    if (mean_out) {
+        const XferSeg seg = {mean_out, t.mean, h->ncells * 3 * sizeof(double)};
+        CK(xfer_down(&seg, 1, h->device, h->stream));
+    }
     CK(cudaStreamSynchronize(h->stream));
     if (out.lost) return fail(ST_ERR_PARCEL_OUTSIDE, "parcel(s) left the mesh in the forward pass");
     if (out.overflow)
@@ -1351,7 +1346,8 @@ int adj_pullback(st_handle* h, int cloud, const st_adjoint_desc* d, const double
                     "st_mean_source_pullback needs a preceding st_mean_source_forward with the "
                     "same cloud and descriptor");
     const int64_t ncomp = h->ncells * 3;
-    CK(cudaMemcpyAsync(t.ybar, cot, ncomp * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    const XferSeg up = {const_cast<double*>(cot), t.ybar, ncomp * sizeof(double)};
+    CK(xfer_up(&up, 1, h->device, h->stream));
     AdjArgs<P, V> a = adj_args<P, V>(h);
     if (!dv0) a.dv0 = nullptr;
     {
@@ -1364,9 +1360,10 @@ int adj_pullback(st_handle* h, int cloud, const st_adjoint_desc* d, const double
     if (!parts.empty())
         CK(cudaMemcpyAsync(parts.data(), t.partials, parts.size() * sizeof(double),
                            cudaMemcpyDeviceToHost, h->stream));
-    if (dv0 && t.n > 0)
-        CK(cudaMemcpyAsync(dv0, t.dv0, (size_t)3 * t.n * sizeof(double), cudaMemcpyDeviceToHost,
-                           h->stream));
+    if (dv0 && t.n > 0) {
+        const XferSeg down = {dv0, t.dv0, (size_t)3 * t.n * sizeof(double)};
+        CK(xfer_down(&down, 1, h->device, h->stream));
+    }
     CK(cudaStreamSynchronize(h->stream));
     double sa = 0.0, ss = 0.0;  /* fixed order: 256 parcels after 256 parcels */
     for (size_t k = 0; k < parts.size(); k += 2) {
@@ -1448,6 +1445,7 @@ static int create_impl(const st_params* p, const st_mesh_desc* m, int64_t ncells
     DeviceGuard g(device);
 
     st_handle* h = new st_handle();
+    xfer_retain();
     h->p = *p;
     h->m = *m;
     h->tet = tm != nullptr;
@@ -1703,6 +1701,7 @@ int st_destroy(st_handle* h)
     for (auto e : h->pool) cudaEventDestroy(e);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
     delete h;
+    xfer_release();
     return ST_OK;
 }
 
@@ -1887,9 +1886,8 @@ int st_get_order(st_handle* h, int cloud, int32_t* ids)
     if (c.n == 0) return ST_OK;
     if (!ids) return fail(ST_ERR_INVALID_ARGUMENT, "null ids");
     DeviceGuard g(h->device);
-    CK(cudaMemcpyAsync(ids, c.id[c.cur], c.n * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                       h->stream));
-    CK(cudaStreamSynchronize(h->stream));
+    const XferSeg seg = {ids, c.id[c.cur], c.n * sizeof(int32_t)};
+    CK(xfer_down(&seg, 1, h->device, h->stream));
     return ST_OK;
 }
 
@@ -1902,18 +1900,21 @@ static int set_fluid(st_handle* h, const void* U, int elem_bytes, bool device)
         return fail(ST_ERR_INVALID_ARGUMENT, "elem_bytes must be 4 or 8, got %d", elem_bytes);
     DeviceGuard g(h->device);
     const int64_t ncomp = h->ncells * 3;
-    const cudaMemcpyKind kind = device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    if ((size_t)elem_bytes == h->vsz) {
-        CK(cudaMemcpyAsync(h->dU, U, ncomp * elem_bytes, kind, h->stream));
+    const bool same = (size_t)elem_bytes == h->vsz;
+    if (!same && (rc = ensure_stage(h, ncomp * elem_bytes))) return rc;
+    void* const dst = same ? h->dU : h->dstage;
+    if (device) {
+        CK(cudaMemcpyAsync(dst, U, ncomp * elem_bytes, cudaMemcpyDeviceToDevice, h->stream));
     } else {
-        if ((rc = ensure_stage(h, ncomp * elem_bytes))) return rc;
-        CK(cudaMemcpyAsync(h->dstage, U, ncomp * elem_bytes, kind, h->stream));
+        const XferSeg seg = {const_cast<void*>(U), dst, (size_t)(ncomp * elem_bytes)};
+        CK(xfer_up(&seg, 1, h->device, h->stream));
+    }
+    if (!same) {
         ProfScope ps(h, ST_KERNEL_OTHER);
         if (elem_bytes == 8) CK(launch_f64_to_f32((const double*)h->dstage, (float*)h->dU, ncomp, h->stream));
         else CK(launch_f32_to_f64((const float*)h->dstage, (double*)h->dU, ncomp, h->stream));
         h->launches += 1;
     }
-    if (!device) CK(cudaStreamSynchronize(h->stream));
     return ST_OK;
 }
 
@@ -1939,24 +1940,20 @@ int st_step(st_handle* h, double dt, double fluid_scale)
     return DISPATCH(h, do_step, h, dt, fluid_scale);
 }
 
-static int copy_source(st_handle* h, int cloud, void* S, int elem_bytes, bool sync)
+static int copy_source(st_handle* h, int cloud, void* S, int elem_bytes)
 {
     const int64_t ncomp = h->ncells * 3;
-    const double* src = h->dsrc + (int64_t)cloud * h->stride;
+    double* src = h->dsrc + (int64_t)cloud * h->stride;
     int rc;
     if ((rc = join_fin(h))) return rc;
-    if (elem_bytes == 8) {
-        CK(cudaMemcpyAsync(S, src, ncomp * 8, cudaMemcpyDeviceToHost, h->stream));
-    } else {
+    if (elem_bytes != 8) {
         if ((rc = ensure_stage(h, ncomp * 4))) return rc;
-        {
-            ProfScope ps(h, ST_KERNEL_OTHER);
-            CK(launch_f64_to_f32(src, (float*)h->dstage, ncomp, h->stream));
-            h->launches += 1;
-        }
-        CK(cudaMemcpyAsync(S, h->dstage, ncomp * 4, cudaMemcpyDeviceToHost, h->stream));
+        ProfScope ps(h, ST_KERNEL_OTHER);
+        CK(launch_f64_to_f32(src, (float*)h->dstage, ncomp, h->stream));
+        h->launches += 1;
     }
-    if (sync) CK(cudaStreamSynchronize(h->stream));
+    const XferSeg seg = {S, elem_bytes == 8 ? (void*)src : h->dstage, (size_t)(ncomp * elem_bytes)};
+    CK(xfer_down(&seg, 1, h->device, h->stream));
     return ST_OK;
 }
 
@@ -1968,7 +1965,7 @@ int st_get_source(st_handle* h, int cloud, void* S, int elem_bytes)
     if (elem_bytes != 4 && elem_bytes != 8)
         return fail(ST_ERR_INVALID_ARGUMENT, "elem_bytes must be 4 or 8, got %d", elem_bytes);
     DeviceGuard g(h->device);
-    if ((rc = copy_source(h, cloud, S, elem_bytes, true))) return rc;
+    if ((rc = copy_source(h, cloud, S, elem_bytes))) return rc;
     return check_device_errors(h);
 }
 
@@ -2696,7 +2693,7 @@ int st_evolve_cloud(double dt)
     }
     if ((rc = DISPATCH(h, do_step, h, dt, 1.0))) return rc;
     /* source device -> host (A:1148-1152) */
-    if ((rc = copy_source(h, 0, is->second.ptr, is->second.tbytes, true))) return rc;
+    if ((rc = copy_source(h, 0, is->second.ptr, is->second.tbytes))) return rc;
     return check_device_errors(h);
 }
 

@@ -148,26 +148,46 @@ __global__ void __launch_bounds__(256) k_gather(const uint32_t* __restrict__ per
     }
 }
 
-/* out[id[p]] = in[p]: back to the order of st_set_parcels */
+/* Parcels base .. base + m - 1 of the st_set_parcels order as the caller holds them: out =
+ * [7][m] FP64 (x, y, z, u, v, w, d).  inv: k_inverse_ids. */
 template <class P, class V>
-__global__ void k_unpermute(const int32_t* __restrict__ id, int64_t n,
-                            const P* __restrict__ x0, const P* __restrict__ y0,
-                            const P* __restrict__ z0, const V* __restrict__ u0,
-                            const V* __restrict__ v0, const V* __restrict__ w0,
-                            const V* __restrict__ d0, P* __restrict__ x1, P* __restrict__ y1,
-                            P* __restrict__ z1, V* __restrict__ u1, V* __restrict__ v1,
-                            V* __restrict__ w1, V* __restrict__ d1)
+__global__ void k_export(const uint32_t* __restrict__ inv, int64_t base, int64_t m,
+                         const P* __restrict__ x, const P* __restrict__ y,
+                         const P* __restrict__ z, const V* __restrict__ u,
+                         const V* __restrict__ v, const V* __restrict__ w,
+                         const V* __restrict__ d, double* __restrict__ out)
 {
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n;
-         p += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t = id[p];
-        x1[t] = x0[p];
-        y1[t] = y0[p];
-        z1[t] = z0[p];
-        u1[t] = u0[p];
-        v1[t] = v0[p];
-        w1[t] = w0[p];
-        d1[t] = d0[p];
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m;
+         j += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p = inv[base + j];
+        out[j] = (double)x[p];
+        out[m + j] = (double)y[p];
+        out[2 * m + j] = (double)z[p];
+        out[3 * m + j] = (double)u[p];
+        out[4 * m + j] = (double)v[p];
+        out[5 * m + j] = (double)w[p];
+        out[6 * m + j] = (double)d[p];
+    }
+}
+
+/* The reverse: in = [7][m] FP64 into the arrays at base .. base + m - 1, with their ids. */
+template <class P, class V>
+__global__ void k_import(const double* __restrict__ in, int64_t base, int64_t m,
+                         P* __restrict__ x, P* __restrict__ y, P* __restrict__ z,
+                         V* __restrict__ u, V* __restrict__ v, V* __restrict__ w,
+                         V* __restrict__ d, int32_t* __restrict__ id)
+{
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m;
+         j += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t p = base + j;
+        x[p] = (P)in[j];
+        y[p] = (P)in[m + j];
+        z[p] = (P)in[2 * m + j];
+        u[p] = (V)in[3 * m + j];
+        v[p] = (V)in[4 * m + j];
+        w[p] = (V)in[5 * m + j];
+        d[p] = (V)in[6 * m + j];
+        id[p] = (int32_t)p;
     }
 }
 
@@ -464,14 +484,28 @@ cudaError_t sort_cloud(SortBufs<P, V>& b, int cur, int64_t n, const MeshK<P>& me
 }
 
 template <class P, class V>
-cudaError_t unpermute_cloud(SortBufs<P, V>& b, int cur, int64_t n, cudaStream_t s)
+cudaError_t export_order(SortBufs<P, V>& b, int cur, int64_t n, cudaStream_t s)
 {
-    if (n == 0) return cudaSuccess;
-    const int o = 1 - cur;
-    k_unpermute<P, V><<<grid_for(n), 256, 0, s>>>(b.id[cur], n, b.x[cur], b.y[cur], b.z[cur],
-                                                  b.u[cur], b.v[cur], b.w[cur], b.d[cur],
-                                                  b.x[o], b.y[o], b.z[o], b.u[o], b.v[o],
-                                                  b.w[o], b.d[o]);
+    /* the sort's permutation buffer is free between steps: it holds the inverse of the ids */
+    k_inverse_ids<<<grid_for(n), 256, 0, s>>>(b.id[cur], n, b.perm[0]);
+    return cudaGetLastError();
+}
+
+template <class P, class V>
+cudaError_t export_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m, double* out,
+                         cudaStream_t s)
+{
+    k_export<P, V><<<grid_for(m), 256, 0, s>>>(b.perm[0], base, m, b.x[cur], b.y[cur], b.z[cur],
+                                               b.u[cur], b.v[cur], b.w[cur], b.d[cur], out);
+    return cudaGetLastError();
+}
+
+template <class P, class V>
+cudaError_t import_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m, const double* in,
+                         cudaStream_t s)
+{
+    k_import<P, V><<<grid_for(m), 256, 0, s>>>(in, base, m, b.x[cur], b.y[cur], b.z[cur],
+                                               b.u[cur], b.v[cur], b.w[cur], b.d[cur], b.id[cur]);
     return cudaGetLastError();
 }
 
@@ -510,7 +544,11 @@ cudaError_t cells_unpermute(const int32_t* id, const int32_t* cell, int64_t n, i
 #define ST_INST(P, V)                                                                         \
     template cudaError_t sort_cloud<P, V>(SortBufs<P, V>&, int, int64_t, const MeshK<P>&, int, \
                                           int, bool, cudaStream_t, int*);                     \
-    template cudaError_t unpermute_cloud<P, V>(SortBufs<P, V>&, int, int64_t, cudaStream_t); \
+    template cudaError_t export_order<P, V>(SortBufs<P, V>&, int, int64_t, cudaStream_t);      \
+    template cudaError_t export_chunk<P, V>(SortBufs<P, V>&, int, int64_t, int64_t, double*,    \
+                                            cudaStream_t);                                     \
+    template cudaError_t import_chunk<P, V>(SortBufs<P, V>&, int, int64_t, int64_t,             \
+                                            const double*, cudaStream_t);                      \
     template cudaError_t sample_cloud<P, V>(SortBufs<P, V>&, int, int64_t, const MeshK<P>&,    \
                                             const int32_t*, int64_t, double*, int32_t*,        \
                                             cudaStream_t);
