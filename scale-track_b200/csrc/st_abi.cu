@@ -481,17 +481,15 @@ int do_sort_all(st_handle* h)
     return ST_OK;
 }
 
-/* Programmatic dependent launch of the step's kernels: on the library's or a caller's own
- * stream, outside graph capture (a captured graph keeps plain edges) and profiling (its events
- * stand between the kernels).  It hides launch gaps of a few microseconds (1e4 parcels on 20^3
+/* Programmatic dependent launch of the step's kernels: outside graph capture (a captured graph
+ * keeps plain edges) and profiling (its events stand between the kernels).  It hides launch gaps of a few microseconds (1e4 parcels on 20^3
  * cells: 13.0 -> 9.5 us per step, 1e5 on 32^3: 15.0 -> 12.3 us), so only handles with small
  * accumulators use it: with large ones the waiting conversion takes SMs from other handles'
  * steps (64 sources of 64^3 cells, three handles in turn: 1526 against 1358 us per step). */
 bool use_pdl(const st_handle* h)
 {
     return (size_t)h->stride * h->p.n_clouds * h->limbs * 8 <= FINALIZE_CLEAR_BYTES &&
-           !h->capturing && !h->prof && h->stream != nullptr && h->stream != cudaStreamLegacy &&
-           h->stream != cudaStreamPerThread;
+           !h->capturing && !h->prof;
 }
 
 /* The ring or the per-warp kernel for a step of a single cloud of n parcels, unless the

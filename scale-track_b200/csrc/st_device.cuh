@@ -153,6 +153,13 @@ struct Quant {
     float thr_small; /* 2^(SMALL_Q_BITS+L) as float when that is a normal float, else 0 */
 };
 
+/* The scale of a step whose largest deposit's exponent a probe has found (EXP_NONE: there is
+ * no deposit). */
+__device__ __forceinline__ int first_scale(int emax, int H)
+{
+    return emax == EXP_NONE ? -H : emax - H;
+}
+
 /* Quantised deposits below 2^SMALL_Q_BITS in magnitude: a sum of up to eight of them fits in
  * a 32-bit integer (the warp run reduction's 32-bit path). */
 constexpr int SMALL_Q_BITS = 28;

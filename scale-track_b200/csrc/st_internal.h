@@ -109,6 +109,12 @@ struct StepArgs {
     CloudCtl* ctl;              /* [nclouds] */
     int64_t total_tiles;        /* warp tiles (32 parcels) over all clouds */
     CloudK<P, V> one;           /* with one cloud: its descriptor, read from parameter space */
+    /* st_step_noalloc: the scale comes from a probe's largest-deposit exponent and headroom H
+     * (not from ctl), and the probe pass clears the accumulator */
+    const CloudCtl* probed = nullptr;
+    int32_t H = 0;
+    unsigned long long* clear = nullptr;
+    int64_t clear_n = 0;
     int64_t wait_cycles = 0;    /* ring kernels: pipeline-wait limit in SM cycles, 0 = ~1 s;
                                    negative: the failure-detection test (ring_wait_limit) */
 };

@@ -91,6 +91,11 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
         __syncthreads();
     }
     grid_dep_wait();
+    if (DEP == DEP_PROBE && a.clear) {
+        for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < a.clear_n;
+             j += (int64_t)gridDim.x * blockDim.x)
+            a.clear[j] = 0ULL;
+    }
     int cur = -1;
     Quant qp = {0.0, 0.0, 0};
     AmaxT<V> amax = (V)0;
@@ -137,7 +142,12 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
         if (c != cur) {
             if (cur >= 0) flush_ctl<DEP>(a.ctl + cur, lane, amax, ovf, nlost);
             cur = c;
-            if (DET) qp = make_quant(a.ctl[c].L, a.ctl[c].H + QUANT_GROWTH_BITS);
+            if (DET) {
+                if (SINGLE && a.probed)
+                    qp = make_quant(first_scale(a.probed->emax, a.H), a.H + QUANT_GROWTH_BITS);
+                else
+                    qp = make_quant(a.ctl[c].L, a.ctl[c].H + QUANT_GROWTH_BITS);
+            }
         }
         const CloudK<P, V>& cl = SINGLE ? a.one : a.clouds[c];
         const int64_t n = cl.n;
@@ -422,7 +432,7 @@ __global__ void k_set_scale(CloudCtl* ctl, int nclouds)
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < nclouds) {
         int em = ctl[k].emax;
-        ctl[k].L = (em == EXP_NONE) ? -ctl[k].H : em - ctl[k].H;
+        ctl[k].L = first_scale(em, ctl[k].H);
         ctl[k].emax = EXP_NONE;
     }
 }

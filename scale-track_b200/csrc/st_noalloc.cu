@@ -16,35 +16,47 @@
  * be called on a device after it was reset.  Every call ends by reading the control block
  * back and synchronising the stream, so a call cannot be recorded into a CUDA graph: one
  * made on a capturing stream is rejected before anything is launched.  All calls share the
- * one array and it keeps the last call's contents: each call clears the accumulator and
- * control block it needs before use, and calls that overlap on the GPU (other streams or
- * host threads) race on the array.
+ * one array and it keeps the last call's contents: each call clears the accumulator before
+ * use and resets the control blocks of the call after it, and calls that overlap on the GPU
+ * (other streams or host threads) race on the array.
  */
+#include <algorithm>
 #include <climits>
 #include <cstdint>
-#include <cstring>
 #include <mutex>
 
 #include <cuda_runtime.h>
 
 #include "scaletrack.h"
-#include "st_internal.h"
+#include "st_device.cuh"
 
 using namespace st;
 
 namespace {
 
 constexpr int64_t NOALLOC_MAX_CELLS = ST_NOALLOC_MAX_CELLS;  /* include/scaletrack.h */
-constexpr size_t ACC_BYTES = (size_t)NOALLOC_MAX_CELLS * 3 * sizeof(unsigned long long);
-constexpr size_t HDR_BYTES = 512;  /* control block + cloud descriptor, padded */
-static_assert(sizeof(CloudCtl) + sizeof(CloudK<double, float>) <= HDR_BYTES, "header");
+/* the accumulator */
+static __device__ unsigned long long g_st_noalloc_acc[NOALLOC_MAX_CELLS * 3];
 
-/* [0, HDR_BYTES): CloudCtl, then CloudK<double,float>; [HDR_BYTES, ...): accumulator */
-static __device__ __align__(256) unsigned char g_st_noalloc_scratch[HDR_BYTES + ACC_BYTES];
+/* Control blocks of the probe and the step, two sets used in turn: every call's last kernel
+ * resets the set of the next call. */
+struct CtlPair {
+    CloudCtl probe, step;
+};
+#define ST_CTL0 {0, EXP_NONE, 0, 0, 0ULL, 0ULL}
+static __device__ CtlPair g_st_noalloc_ctl[2] = {{ST_CTL0, ST_CTL0}, {ST_CTL0, ST_CTL0}};
+#undef ST_CTL0
 
 constexpr int MAX_DEVICES = 64;
+struct Scratch {
+    CtlPair* ctl = nullptr;
+    unsigned long long* acc = nullptr;
+    int resident = 0;    /* step blocks that stay resident on the device */
+    int next = 0;        /* the control set of the next call */
+    bool dirty = false;  /* a call failed before its last kernel: both sets need a reset */
+};
 std::mutex g_mu;
-unsigned char* g_scratch_addr[MAX_DEVICES] = {nullptr};
+Scratch g_scratch[MAX_DEVICES];
 
 int fail(int code, const char* msg)
 {
@@ -52,32 +64,35 @@ int fail(int code, const char* msg)
     return code;
 }
 
-/* Writes the control block and the cloud descriptor (passed by value: no host copy). */
-__global__ void k_noalloc_init(CloudCtl ctl, CloudK<double, float> cloud, CloudCtl* ctl_dst,
-                               CloudK<double, float>* cloud_dst)
+__device__ __forceinline__ void reset(CtlPair* c)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        *ctl_dst = ctl;
-        *cloud_dst = cloud;
-    }
+    const CloudCtl c0 = {0, EXP_NONE, 0, 0, 0ULL, 0ULL};
+    c->probe = c0;
+    c->step = c0;
 }
 
-/* After the read-only probe: the scale maps the largest deposit of this call to 2^H. */
-__global__ void k_noalloc_scale(CloudCtl* ctl)
+__global__ void k_noalloc_reset(CtlPair* both)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int em = ctl->emax;
-        ctl->L = (em == EXP_NONE) ? -ctl->H : em - ctl->H;
-        ctl->emax = EXP_NONE;
-    }
+    if (threadIdx.x < 2) reset(both + threadIdx.x);
 }
 
-/* Fixed point -> FP64 into the caller's [nCells][3] source (any length, scalar stores). */
-__global__ void k_noalloc_finalize(const unsigned long long* __restrict__ acc,
-                                   const CloudCtl* ctl, double* __restrict__ src,
-                                   int64_t ncomp)
+/* Fixed point -> FP64 into the caller's [nCells][3] source (any length, scalar stores), and
+ * the control set of the next call.
+ *
+ * A call is a chain of three kernels, each launched programmatically behind the one before
+ * (its launch and set-up overlap the previous kernel's end): the probe, which also clears the
+ * accumulator; the step, its scale straight from the probe's control block; the conversion.
+ * What bounds the smallest calls is the chain's latency and the read-back of the control block:
+ * 3001 parcels on 12^3 cells took 48.8 us as a memset and five kernels in stream order with the
+ * occupancy queried on every call, 32.0 us now (a kernel and a read-back alone: 20 us); 1e6 on
+ * 64^3 cells 87.6 -> 78.4 us. */
+__global__ void __launch_bounds__(256) k_noalloc_finalize(
+    const unsigned long long* __restrict__ acc, const CtlPair* ctl, CtlPair* next, int H,
+    double* __restrict__ src, int64_t ncomp)
 {
-    const int L = ctl->L;
+    grid_dep_wait();
+    if (blockIdx.x == 0 && threadIdx.x == 0) reset(next);
+    const int L = first_scale(ctl->probe.emax, H);
     const int k1 = L / 2, k2 = L - L / 2;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < ncomp;
          j += (int64_t)gridDim.x * blockDim.x) {
@@ -145,36 +160,40 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
                         "st_step_noalloc synchronises its stream and cannot be captured into a "
                         "CUDA graph");
     }
-    unsigned char* base;
+    Scratch sc;
     {
         std::lock_guard<std::mutex> lk(g_mu);
-        if (!g_scratch_addr[dev]) {
-            void* ptr = nullptr;
-            cudaError_t e = cudaGetSymbolAddress(&ptr, g_st_noalloc_scratch);
-            if (e != cudaSuccess || !ptr)
-                return fail(ST_ERR_CUDA, cudaGetErrorString(e));
-            g_scratch_addr[dev] = static_cast<unsigned char*>(ptr);
+        Scratch& g = g_scratch[dev];
+        if (!g.acc) {
+            void *pc = nullptr, *pa = nullptr;
+            cudaError_t e = cudaGetSymbolAddress(&pc, g_st_noalloc_ctl);
+            if (e == cudaSuccess) e = cudaGetSymbolAddress(&pa, g_st_noalloc_acc);
+            if (e != cudaSuccess || !pc || !pa) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
+            int nsm = 148;
+            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+            const int occ = step_max_active_blocks<double, float>(DEP_DET1, 256);
+            g.resident = nsm * (occ < 1 ? 1 : occ);
+            g.ctl = static_cast<CtlPair*>(pc);
+            g.acc = static_cast<unsigned long long*>(pa);
         }
-        base = g_scratch_addr[dev];
+        sc = g;
+        g.next ^= 1;
+        g.dirty = true;   /* until this call's last kernel is on its way */
     }
-    CloudCtl* ctl = reinterpret_cast<CloudCtl*>(base);
-    CloudK<double, float>* cloud =
-        reinterpret_cast<CloudK<double, float>*>(base + sizeof(CloudCtl));
-    unsigned long long* acc = reinterpret_cast<unsigned long long*>(base + HDR_BYTES);
+    CtlPair* const ctl = sc.ctl + sc.next;
+    unsigned long long* const acc = sc.acc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int64_t ncomp = ncells * 3;
 
-    CloudCtl c0;
-    std::memset(&c0, 0, sizeof c0);
-    c0.emax = EXP_NONE;
     const int64_t bound = n * (int64_t)p->n_substeps > 2 ? n * (int64_t)p->n_substeps : 2;
-    c0.H = 62 - QUANT_GROWTH_BITS - quant_nbits(bound);
+    const int H = 62 - QUANT_GROWTH_BITS - quant_nbits(bound);
     CloudK<double, float> ck;
     ck.x = x; ck.y = y; ck.z = z; ck.u = u; ck.v = v; ck.w = w; ck.d = d;
     ck.n = n;
     ck.tile0 = 0;
     ck.acc = acc;
     ck.src = nullptr;
+    ck.cell = nullptr;
 
     StepArgs<double, float> a;
     for (int k = 0; k < 3; ++k) {
@@ -199,36 +218,47 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
     split_fluid_scale<double, float>(fluid_scale, a.fscale, a.fscale_lo);
     a.nclouds = 1;
     a.U = U;
-    a.clouds = cloud;
-    a.ctl = ctl;
+    a.clouds = nullptr;   /* one cloud: its descriptor is in the kernel parameters */
+    a.ctl = &ctl->step;
     a.total_tiles = (n + WARP_TILE - 1) / WARP_TILE;
     a.one = ck;
 
     cudaError_t e;
-    if ((e = cudaMemsetAsync(acc, 0, (size_t)ncomp * sizeof(unsigned long long), s)) != cudaSuccess)
-        return fail(ST_ERR_CUDA, cudaGetErrorString(e));
-    k_noalloc_init<<<1, 32, 0, s>>>(c0, ck, ctl, cloud);
-    if ((e = cudaGetLastError()) != cudaSuccess) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
-    if (n > 0) {
-        int nsm = 148, occ = 1;
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        occ = step_max_active_blocks<double, float>(DEP_DET1, 256);
-        if (occ < 1) occ = 1;
-        int64_t need = (a.total_tiles + 7) / 8;
-        int grid = (int)(need < (int64_t)nsm * occ ? need : (int64_t)nsm * occ);
-        if (grid < 1) grid = 1;
-        if ((e = launch_step<double, float>(a, DEP_PROBE, grid, 256, s)) != cudaSuccess)
-            return fail(ST_ERR_CUDA, cudaGetErrorString(e));
-        k_noalloc_scale<<<1, 32, 0, s>>>(ctl);
-        if ((e = launch_step<double, float>(a, DEP_DET1, grid, 256, s)) != cudaSuccess)
+    if (sc.dirty) {
+        k_noalloc_reset<<<1, 32, 0, s>>>(sc.ctl);
+        if ((e = cudaGetLastError()) != cudaSuccess)
             return fail(ST_ERR_CUDA, cudaGetErrorString(e));
     }
-    int fgrid = (int)((ncomp + 255) / 256 < 148 * 8 ? (ncomp + 255) / 256 : 148 * 8);
-    k_noalloc_finalize<<<fgrid, 256, 0, s>>>(acc, ctl, source, ncomp);
-    if ((e = cudaGetLastError()) != cudaSuccess) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
+    {
+        /* with no parcels the probe still clears the accumulator */
+        const int64_t need = (std::max(a.total_tiles, (ncomp + 31) / 32) + 7) / 8;
+        StepArgs<double, float> probe = a;
+        probe.ctl = &ctl->probe;
+        probe.clear = acc;
+        probe.clear_n = ncomp;
+        e = launch_step<double, float>(probe, DEP_PROBE, (int)std::min<int64_t>(need, sc.resident),
+                                       256, s, false);
+        if (e != cudaSuccess) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
+    }
+    if (n > 0) {
+        const int64_t need = (a.total_tiles + 7) / 8;
+        a.probed = &ctl->probe;
+        a.H = H;
+        e = launch_step<double, float>(a, DEP_DET1, (int)std::min<int64_t>(need, sc.resident), 256,
+                                       s, true);
+        if (e != cudaSuccess) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
+    }
+    const int fgrid = (int)std::min<int64_t>((ncomp + 255) / 256, 148 * 8);
+    e = launch_kernel(true, k_noalloc_finalize, dim3(fgrid), dim3(256), 0, s, acc, ctl,
+                      sc.ctl + (sc.next ^ 1), H, source, ncomp);
+    if (e != cudaSuccess) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        g_scratch[dev].dirty = false;
+    }
 
     CloudCtl out;
-    if ((e = cudaMemcpyAsync(&out, ctl, sizeof out, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
+    if ((e = cudaMemcpyAsync(&out, &ctl->step, sizeof out, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return fail(ST_ERR_CUDA, cudaGetErrorString(e));
     if (out.lost) return fail(ST_ERR_PARCEL_OUTSIDE, "parcel(s) could not be located in the mesh");

@@ -76,3 +76,60 @@ def test_small_cloud_paths_agree(prec, nsub, n):
     assert r["status"] == 0
     for x, y in zip(g, (r["xyz"], r["uvw"], r["cells"], r["src_quant"])):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("npcl", [0, 1, 33, 3001])
+def test_noalloc_calls_in_a_row(npcl):
+    """The allocation-free step uses two control sets in turn, each reset by the call before:
+    five calls in a row, one of them with a parcel outside the mesh (its error is its own) and
+    on alternating streams, each give the source of a fresh handle that steps the same parcels
+    (the scale comes from each call's own largest deposit, as a fresh handle's first step)."""
+    import ctypes
+    import torch
+    n = 9
+    xyz, uvw, d = workload.parcels(max(npcl, 1), 90)
+    xyz, uvw, d = xyz[:, :npcl], uvw[:, :npcl], d[:npcl]
+    U = workload.tgv_field(n, dtype=np.float32)
+    prm = st.params(mu_c=workload.MU_F, rho_c=workload.RHO_F, rho_d=workload.RHO_P,
+                    drag_model="schiller_naumann", precision="mixed", n_substeps=1)
+    mesh = st.mesh_desc(n, 0.0, workload.L_BOX)
+    dev = torch.device("cuda", 0)
+    X = [torch.tensor(a, dtype=torch.float64, device=dev) for a in xyz]
+    V = [torch.tensor(a, dtype=torch.float32, device=dev) for a in uvw]
+    D = torch.tensor(d, dtype=torch.float32, device=dev)
+    Ud = torch.tensor(U, device=dev)
+    S = torch.full((n ** 3, 3), float("nan"), dtype=torch.float64, device=dev)
+    streams = [torch.cuda.default_stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+
+    def call(k):
+        p = ctypes.c_void_p
+        return st.lib().st_step_noalloc(
+            ctypes.byref(prm), ctypes.byref(mesh), npcl, *[p(t.data_ptr() or None) for t in X],
+            *[p(t.data_ptr() or None) for t in V], p(D.data_ptr() or None), p(Ud.data_ptr()),
+            p(S.data_ptr()), workload.DT, 1.0, p(streams[k % 2].cuda_stream))
+
+    for k in range(5):
+        if npcl > 1 and k == 2:      # a call that reports a lost parcel
+            keep = X[0][0].item()
+            X[0][0] = 2.5 * workload.L_BOX
+            torch.cuda.synchronize()
+            assert call(k) == st.ST_ERR_PARCEL_OUTSIDE
+            X[0][0] = keep
+            torch.cuda.synchronize()
+            continue
+        ref = np.zeros((n ** 3, 3))
+        if npcl:
+            x = np.stack([t.cpu().numpy() for t in X])
+            v = np.stack([t.cpu().numpy().astype(np.float64) for t in V])
+            with st.ParcelTracker(prm, mesh) as h:
+                h.set_parcels(x, v, d)
+                h.set_fluid_velocity(U)
+                h.step(workload.DT)
+                ref = h.get_source()
+                px, pv, _ = h.get_parcels()
+        assert call(k) == st.ST_OK, st.last_error()
+        assert np.array_equal(S.cpu().numpy(), ref)
+        if npcl:
+            assert np.array_equal(np.stack([t.cpu().numpy() for t in X]), px)
+            assert np.array_equal(np.stack([t.cpu().numpy() for t in V]).astype(np.float64), pv)
