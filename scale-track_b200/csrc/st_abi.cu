@@ -644,6 +644,7 @@ int do_step(st_handle* h, double dt, double fscale, int phase = PH_ALL)
     a.dtP = (P)dt / (P)h->p.n_substeps;
     a.dtV = (V)a.dtP;
     split_fluid_scale<P, V>(fscale, a.fscale, a.fscale_lo);
+    set_locate_bounds(a);
     a.nclouds = h->p.n_clouds;
     a.U = (const V*)h->dU;
     a.clouds = h->capturing
@@ -1122,6 +1123,7 @@ int graph_capture(st_handle* h, int n, double dt, const double* fs)
         a.dtP = (P)dt / (P)h->p.n_substeps;
         a.dtV = (V)a.dtP;
         split_fluid_scale<P, V>(fs ? fs[0] : 1.0, a.fscale, a.fscale_lo);
+        set_locate_bounds(a);
         a.nclouds = h->p.n_clouds;
         a.U = (const V*)h->dU;
         a.clouds = (const CloudK<P, V>*)h->dclouds;

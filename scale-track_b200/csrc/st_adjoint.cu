@@ -79,7 +79,7 @@ struct AdjLocal {
 template <class V>
 __device__ __forceinline__ V adj_pow(V Re)
 {
-    if (sizeof(V) == 4) return (V)st_pow0687f((float)Re);
+    if (sizeof(V) == 4) return (V)pow0687f((float)Re);
     return (V)st_pow0687((double)Re);
 }
 

@@ -67,14 +67,35 @@ __device__ __forceinline__ void pow_tab_fill()
     }
 }
 
+/* Exponent and first factor of st_pow0687f_mant for a positive normal x by integers alone;
+ * false for every other x.  With 0x3f3504f4 the float after sqrt(1/2) rounded down, bits -
+ * 0x3f3504f4 has the exponent e of x = 2^e m, sqrt(1/2) < m <= sqrt(2), in its upper bits, and
+ * subtracting e from the exponent field leaves m. */
+__device__ __forceinline__ bool pow0687f_split(float x, int& e, float& p)
+{
+    const uint32_t b = __float_as_uint(x);
+    const int32_t r = (int32_t)(b - 0x3f3504f4u);
+    e = r >> 23;
+    p = st_pow0687f_poly(__uint_as_float(b - ((uint32_t)r & 0xff800000u)) - 1.0f);
+    return b - 0x00800000u < 0x7f000000u;
+}
+
+/* st_pow0687f bit for bit: with the table, and with the exponent factor's polynomial */
 __device__ __forceinline__ float pow0687f_tab(float x)
 {
-    if (!(x > 0.0f)) return x != x ? x : 0.0f;
-    if ((__float_as_uint(x) >> 23) == 0xffu) return x;   /* +inf */
     int e;
-    const float p = st_pow0687f_mant(x, &e);
+    float p;
+    if (!pow0687f_split(x, e, p)) return st_pow0687f(x);   /* 0, subnormal, inf, NaN, < 0 */
     const float2 qs = s_pow_tab[e - POW_TAB_EMIN];
     return (p * qs.x) * qs.y;
+}
+__device__ __forceinline__ float pow0687f(float x)
+{
+    int e;
+    float p, q, s2k;
+    if (!pow0687f_split(x, e, p)) return st_pow0687f(x);
+    st_pow0687f_efac(e, &q, &s2k);
+    return (p * q) * s2k;
 }
 
 /* slip with the product of the raw cell value and the low part of the fluid factor given
@@ -261,20 +282,21 @@ __device__ __forceinline__ void deposit_direct(const V dep[3], int64_t cell0,
                                                unsigned long long* acc, double* src,
                                                const Quant& qp, AmaxT<V>& amax, unsigned& ovf)
 {
+    if constexpr (DEP == DEP_ATOMIC) {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        if (DEP == DEP_ATOMIC) {
+        for (int c = 0; c < 3; ++c)
             if (dep[c] != (V)0) red_add(src + 3 * cell0 + c, (double)dep[c]);
-        } else {
-            long long q = quantize(dep[c], qp, amax, ovf);
-            if (DEP == DEP_DET1) {
-                if (q) red_add(acc + 3 * cell0 + c, (unsigned long long)q);
-            } else if (DEP == DEP_DET2) {
-                if (q) {
-                    red_add(acc + 2 * (3 * cell0 + c), (unsigned long long)(q >> 32));
-                    red_add(acc + 2 * (3 * cell0 + c) + 1,
-                              (unsigned long long)q & 0xffffffffULL);
-                }
+    } else {
+        long long q[3];
+        quantize3(dep, qp, amax, ovf, q);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if (!q[c]) continue;
+            if constexpr (DEP == DEP_DET1) {
+                red_add(acc + 3 * cell0 + c, (unsigned long long)q[c]);
+            } else {
+                red_add(acc + 2 * (3 * cell0 + c), (unsigned long long)(q[c] >> 32));
+                red_add(acc + 2 * (3 * cell0 + c) + 1, (unsigned long long)q[c] & 0xffffffffULL);
             }
         }
     }

@@ -108,6 +108,12 @@ struct StepArgs {
     const CloudK<P, V>* clouds; /* [nclouds] device array */
     CloudCtl* ctl;              /* [nclouds] */
     int64_t total_tiles;        /* warp tiles (32 parcels) over all clouds */
+    /* shortcuts of the relocation (set_locate_bounds): a velocity component below vsafe moves
+     * a parcel by less than half a cell per step; cells per velocity and substep, and the
+     * half width of the part of a cell where the FP32 cell coordinate decides (0: never) */
+    V vsafe[3];
+    float cdt[3];
+    float half;
     CloudK<P, V> one;           /* with one cloud: its descriptor, read from parameter space */
     /* st_step_noalloc: the scale comes from a probe's largest-deposit exponent and headroom H
      * (not from ctl), and the probe pass clears the accumulator */
@@ -118,6 +124,41 @@ struct StepArgs {
     int64_t wait_cycles = 0;    /* ring kernels: pipeline-wait limit in SM cycles, 0 = ~1 s;
                                    negative: the failure-detection test (ring_wait_limit) */
 };
+
+/* Sets vsafe, cdt and half from the mesh, the substep and the substep count.  u is the unit
+ * roundoff of the positions, X the largest coordinate of the mesh (with a cell of margin), N
+ * the cells of an axis, all bounds in cells:
+ *   one update x + v dt errs by at most 2 u X rD, the fractional coordinate (x - o) rD as the
+ *   kernels form it by 4 u N against its exact value;
+ * vsafe: a parcel at least one cell away from both ends of every axis that moves by less than
+ * 0.5 (1 + 2^-20), with those errors below 0.25, stays inside the mesh.
+ * half: the FP32 cell coordinate starts within 2^-24, and each substep adds 2^-23 + 2^-24 (the
+ * product, the sum; a move of a cell or more leaves the decided part) and the update's error.
+ * With the total below 2^-11, a coordinate within [2^-10, 1 - 2^-10] has the same floor as the
+ * kernels' own. */
+template <class P, class V>
+inline void set_locate_bounds(StepArgs<P, V>& a)
+{
+    const double u = sizeof(P) == 8 ? 0x1p-53 : 0x1p-24;
+    double step = 0.0, form = 0.0;   /* worst axis */
+    for (int k = 0; k < 3; ++k) {
+        const double rD = (double)a.mesh.rD[k], o = (double)a.mesh.origin[k];
+        const double e = o + (a.mesh.N[k] + 1.0) / rD;
+        const double X = (o < 0 ? -o : o) > (e < 0 ? -e : e) ? (o < 0 ? -o : o) : (e < 0 ? -e : e);
+        const double s = 2.0 * u * (X + 1.0 / rD) * rD, f = 4.0 * u * (a.mesh.N[k] + 2.0);
+        step = s > step ? s : step;
+        form = f > form ? f : form;
+        const double c = (double)a.dtP * rD;
+        a.cdt[k] = (float)c;
+        a.vsafe[k] = (V)(0.5 / c);
+        if (!(a.vsafe[k] > (V)0 && a.vsafe[k] < (V)1e30)) a.vsafe[k] = (V)0;
+        if (!(a.cdt[k] > 1e-30f && a.cdt[k] < 1e30f)) step = 1.0;
+    }
+    if (!(step + form < 0.25))
+        for (int k = 0; k < 3; ++k) a.vsafe[k] = (V)0;
+    const double err = 0x1p-23 + a.phys.nsub * (0x1.8p-23 + step) + form;
+    a.half = err < 0x1p-11 ? 0.5f - 0x1p-10f : 0.0f;
+}
 
 /* Unstructured tetrahedral mesh (st_tet.cu). */
 struct TetMeshK {

@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
     __shared__ unsigned long long dep_ws[8][dep_ws_words<DEP, V>];
     unsigned long long* const ws = dep_ws[threadIdx.x >> 5];
     grid_dep_launch();
-    if (!ONE) {   /* the table of x^0.687 serves the multi-substep loop */
+    if (!ONE && sizeof(V) == 4 && a.phys.drag != 0) {   /* the table of x^0.687 serves the multi-substep loop */
         pow_tab_fill();
         __syncthreads();
     }
@@ -97,7 +97,9 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
             a.clear[j] = 0ULL;
     }
     int cur = -1;
-    Quant qp = {0.0, 0.0, 0};
+    /* in shared memory: nine registers less through the substeps */
+    __shared__ Quant s_qp[8];
+    Quant& qp = s_qp[threadIdx.x >> 5];
     AmaxT<V> amax = (V)0;
     unsigned ovf = 0, nlost = 0;
 
@@ -143,10 +145,13 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
             if (cur >= 0) flush_ctl<DEP>(a.ctl + cur, lane, amax, ovf, nlost);
             cur = c;
             if (DET) {
-                if (SINGLE && a.probed)
-                    qp = make_quant(first_scale(a.probed->emax, a.H), a.H + QUANT_GROWTH_BITS);
-                else
-                    qp = make_quant(a.ctl[c].L, a.ctl[c].H + QUANT_GROWTH_BITS);
+                const Quant q = SINGLE && a.probed
+                                    ? make_quant(first_scale(a.probed->emax, a.H),
+                                                 a.H + QUANT_GROWTH_BITS)
+                                    : make_quant(a.ctl[c].L, a.ctl[c].H + QUANT_GROWTH_BITS);
+                __syncwarp();
+                if (lane == 0) qp = q;
+                __syncwarp();
             }
         }
         const CloudK<P, V>& cl = SINGLE ? a.one : a.clouds[c];
@@ -164,16 +169,16 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
         if (AHEAD) R = RN;
         /* phase 2: start cells (A:1286) and raw cell velocities (A:1288; the fluid factor is
          * applied in the slip) */
-        int32_t pI[SLICES];
+        LocK st0[SLICES];
         V Ur[SLICES][3];
 #pragma unroll
         for (int s = 0; s < SLICES; ++s) {
-            pI[s] = 0;
+            st0[s].posI = 0;
             if (base + 32 * s < n) {
                 bool bad = false;
-                LocK l0 = locate(a.mesh, X[s], Y[s], Z[s], bad);
+                const LocK l0 = locate(a.mesh, X[s], Y[s], Z[s], bad);
                 if (!bad && l0.part == 1) {
-                    pI[s] = l0.posI;
+                    st0[s] = l0;
                     const V* Uc = a.U + 3 * (int64_t)(l0.posI - 1);
                     Ur[s][0] = __ldg(Uc);
                     Ur[s][1] = __ldg(Uc + 1);
@@ -189,15 +194,16 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
             const int64_t i = base + 32 * s;
             int32_t key = -1;
             V dep[3] = {(V)0, (V)0, (V)0};
-            if (pI[s] > 0) {
+            if (st0[s].posI > 0) {
                 P pos[3] = {X[s], Y[s], Z[s]};
                 V vel[3] = {Uv[s], Vv[s], Wv[s]};
                 bool lost = false;
                 if (ONE) {
-                    evolve_one<P, V>(a, pos, vel, D[s] * a.phys.dscale, pI[s], Ur[s], lost, dep);
-                    key = pI[s] - 1;
+                    evolve_one<P, V, false>(a, pos, vel, D[s] * a.phys.dscale, st0[s].posI,
+                                     interior(a.mesh, st0[s]), Ur[s], lost, dep);
+                    key = st0[s].posI - 1;
                 } else {
-                    evolve_parcel<P, V, DEP>(a, pos, vel, D[s] * a.phys.dscale, pI[s], Ur[s],
+                    evolve_parcel<P, V, DEP>(a, pos, vel, D[s] * a.phys.dscale, st0[s], Ur[s],
                                              acc, src, qp, amax, ovf, lost, key, dep);
                 }
                 if (lost) {

@@ -216,6 +216,7 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
     a.dtP = dt / (double)p->n_substeps;
     a.dtV = (float)a.dtP;
     split_fluid_scale<double, float>(fluid_scale, a.fscale, a.fscale_lo);
+    set_locate_bounds(a);
     a.nclouds = 1;
     a.U = U;
     a.clouds = nullptr;   /* one cloud: its descriptor is in the kernel parameters */

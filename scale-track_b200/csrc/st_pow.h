@@ -189,6 +189,19 @@ ST_HD float st_fmaf(float a, float b, float c)
  * tests check this against a double-precision reference).
  *
  * st_pow0687f_mant: for finite x > 0, the first factor p and the exponent e. */
+ST_HD float st_pow0687f_poly(float t)                 /* (1 + t)^0.687 */
+{
+    float p = -0x1.921f0ep-8f;
+    p = st_fmaf(p, t, 0x1.68372ap-7f);
+    p = st_fmaf(p, t, -0x1.b6bb7ep-7f);
+    p = st_fmaf(p, t, 0x1.2657a8p-6f);
+    p = st_fmaf(p, t, -0x1.bd5c3ap-6f);
+    p = st_fmaf(p, t, 0x1.817e2ap-5f);
+    p = st_fmaf(p, t, -0x1.b862bep-4f);
+    p = st_fmaf(p, t, 0x1.5fbe76p-1f);
+    return st_fmaf(p, t, 1.0f);
+}
+
 ST_HD float st_pow0687f_mant(float x, int* ep)
 {
     uint32_t b = st_bits_of_f(x);
@@ -204,16 +217,7 @@ ST_HD float st_pow0687f_mant(float x, int* ep)
         m = m * 0.5f;
         e += 1;
     }
-    const float t = m - 1.0f;
-    float p = -0x1.921f0ep-8f;
-    p = st_fmaf(p, t, 0x1.68372ap-7f);
-    p = st_fmaf(p, t, -0x1.b6bb7ep-7f);
-    p = st_fmaf(p, t, 0x1.2657a8p-6f);
-    p = st_fmaf(p, t, -0x1.bd5c3ap-6f);
-    p = st_fmaf(p, t, 0x1.817e2ap-5f);
-    p = st_fmaf(p, t, -0x1.b862bep-4f);
-    p = st_fmaf(p, t, 0x1.5fbe76p-1f);
-    p = st_fmaf(p, t, 1.0f);
+    const float p = st_pow0687f_poly(m - 1.0f);
     *ep = e;                                       /* -149 <= e <= 128 */
     return p;
 }

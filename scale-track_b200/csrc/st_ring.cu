@@ -57,12 +57,14 @@ __device__ __forceinline__ void ring_slices(const StepArgs<P, V>& a, P* xs, P* y
 {
     P X[RING_SPW], Y[RING_SPW], Z[RING_SPW];
     V Uv[RING_SPW], Vv[RING_SPW], Wv[RING_SPW], D[RING_SPW];
-    int32_t pI[RING_SPW];
+    LocK st0[RING_SPW];
+    bool inner[RING_SPW];
     V Ur[RING_SPW][3];
 #pragma unroll
     for (int s = 0; s < RING_SPW; ++s) {
         const int j = j0 + 32 * s;
-        pI[s] = 0;
+        st0[s].posI = 0;
+        inner[s] = false;
         if (!GLOBAL || j < nvalid) {
             X[s] = ring_ld<GLOBAL>(xs + j);
             Y[s] = ring_ld<GLOBAL>(ys + j);
@@ -72,9 +74,14 @@ __device__ __forceinline__ void ring_slices(const StepArgs<P, V>& a, P* xs, P* y
             Wv[s] = ring_ld<GLOBAL>(ws + j);
             D[s] = ring_ld<GLOBAL>(ds + j);
             bool bad = false;
-            LocK l0 = locate(a.mesh, X[s], Y[s], Z[s], bad);                  /* A:1286 */
+            const LocK l0 = locate(a.mesh, X[s], Y[s], Z[s], bad);            /* A:1286 */
             if (!bad && l0.part == 1) {
-                pI[s] = l0.posI;
+                if (ONE) {
+                    st0[s].posI = l0.posI;
+                    inner[s] = interior(a.mesh, l0);
+                } else {
+                    st0[s] = l0;
+                }
                 const V* Uc = a.U + 3 * (int64_t)(l0.posI - 1);                /* A:1288 */
                 Ur[s][0] = __ldg(Uc);
                 Ur[s][1] = __ldg(Uc + 1);
@@ -89,15 +96,16 @@ __device__ __forceinline__ void ring_slices(const StepArgs<P, V>& a, P* xs, P* y
         const int j = j0 + 32 * s;
         int32_t key = -1;
         V dep[3] = {(V)0, (V)0, (V)0};
-        if (pI[s] > 0) {
+        if (st0[s].posI > 0) {
             P pos[3] = {X[s], Y[s], Z[s]};
             V vel[3] = {Uv[s], Vv[s], Wv[s]};
             bool lost = false;
             if (ONE) {
-                evolve_one<P, V>(a, pos, vel, D[s] * a.phys.dscale, pI[s], Ur[s], lost, dep);
-                key = pI[s] - 1;
+                evolve_one<P, V, true>(a, pos, vel, D[s] * a.phys.dscale, st0[s].posI, inner[s], Ur[s],
+                                 lost, dep);
+                key = st0[s].posI - 1;
             } else {
-                evolve_parcel<P, V, DEP>(a, pos, vel, D[s] * a.phys.dscale, pI[s], Ur[s], acc,
+                evolve_parcel<P, V, DEP>(a, pos, vel, D[s] * a.phys.dscale, st0[s], Ur[s], acc,
                                          src, qp, amax, ovf, lost, key, dep);
             }
             if (lost) {
@@ -153,7 +161,7 @@ __global__ void __launch_bounds__(HexShapeOf<V>::type::THREADS, 1)
     HexRing<P, V, DEP, ONE> step{a, DET ? a.one.acc : nullptr,
                                  DEP == DEP_ATOMIC ? a.one.src : nullptr, qp, lane, amax, ovf,
                                  nlost, dep_ws[min(threadIdx.x >> 5, HexShape::CONS - 1)]};
-    if (!ONE) pow_tab_fill();   /* ring_block synchronises the block before any step */
+    if (sizeof(V) == 4 && a.phys.drag != 0) pow_tab_fill();   /* ring_block synchronises the block before any step */
     ring_emax_init();
     if (!ring_block<HexShape, P, V, false>(a.one, a.ctl, step, a.wait_cycles)) return;
     flush_ctl<DEP>(a.ctl, lane, amax, ovf, nlost, DEP != DEP_ATOMIC ? &s_ring_emax : nullptr);

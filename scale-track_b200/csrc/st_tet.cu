@@ -242,7 +242,7 @@ __device__ __forceinline__ void tet_parcel(const TetStepArgs<V>& a, int nsub, do
             V mag = st_sqrt((du[0] * du[0] + du[1] * du[1]) + du[2] * du[2]);
             V Re = (mag * d) * ph.rnu;
             V pw;
-            if (sizeof(V) == 4) pw = (V)st_pow0687f((float)Re);
+            if (sizeof(V) == 4) pw = (V)pow0687f((float)Re);
             else pw = (V)st_pow0687((double)Re);
             V g = f * ((V)1 + (V)0.15 * pw);
 #pragma unroll
