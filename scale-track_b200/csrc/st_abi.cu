@@ -501,17 +501,15 @@ bool use_pdl(const st_handle* h)
  *   hex, FP32 and mixed:  1e4 15.9 / 9.5   1e5 14.6 / 12.3   1.5e6 41.1 / 41.0   4e6 84.5 / 92.6
  *   hex, FP64:   1e5 17.7 / 15.0   4e5 25.2 / 24.9   5e5 30.1 / 32.1   4e6 141 / 151
  *   hex, mixed, ten substeps:  1e6 118 / 99   4e6 386 / 333   1e7 987 / 859
- *   tet, mixed:  2e5 23.0 / 21.5   4e5 29.0 / 29.4   1e6 47.5 / 50.2; three substeps:
- *                2e5 37.7 / 35.9   1e6 80.5 / 87.3
- *   tet, FP64:   4e5 35.6 / 35.8   7e5 64.6 / 64.4   1.5e6 105 / 108; three substeps:
- *                1.5e6 190 / 186
+ *   tet, mixed:  2e5 22.0 / 20.4   4e5 27.1 / 27.6   1e6 43.6 / 46.2; three substeps: 1e6 73 / 78
+ *   tet, FP64:   4e5 33.6 / 35.3   1e6 75.2 / 79.4   2e6 123 / 131
  * A wait limit set by the caller is about the ring's waits: the ring then runs at any size. */
 bool use_ring(const st_handle* h, int64_t n)
 {
     if (h->kernel >= 0) return h->kernel == ST_STEP_KERNEL_RING;
     if (h->wait_cycles != 0) return true;
     const bool fp64 = h->p.precision == ST_PREC_FP64;
-    if (h->tet) return n >= (fp64 ? 1000000 : 300000);
+    if (h->tet) return n >= 300000;
     return h->p.n_substeps == 1 && n >= (fp64 ? 450000 : 1500000);
 }
 

@@ -113,22 +113,38 @@ __device__ __forceinline__ int tet_step32(const TetMeshK& m, int32_t t, const fl
     float s[4], e[4];
     bool in = true;
 #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-        const float4 q = __ldg(pl + f);
-        s[f] = ((q.x * x[0] + q.y * x[1]) + q.z * x[2]) - q.w;
-        e[f] = 4.0e-7f * (((fabsf(q.x) + fabsf(q.y)) + fabsf(q.z)) * m.xmax + fabsf(q.w)) +
-               1.0e-37f;
-        in = in && (s[f] < -e[f]);
+    for (int h = 0; h < 2; ++h) {
+        /* two planes in one 32-byte load */
+        float q[8];
+        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(q[0]), "=f"(q[1]), "=f"(q[2]), "=f"(q[3]), "=f"(q[4]), "=f"(q[5]), "=f"(q[6]),
+              "=f"(q[7])
+            : "l"(__cvta_generic_to_global(pl + 2 * h)));
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+            const int f = 2 * h + g;
+            const float* p = q + 4 * g;
+            s[f] = ((p[0] * x[0] + p[1] * x[1]) + p[2] * x[2]) - p[3];
+            e[f] = 4.0e-7f * (((fabsf(p[0]) + fabsf(p[1])) + fabsf(p[2])) * m.xmax +
+                              fabsf(p[3])) + 1.0e-37f;
+            in = in && (s[f] < -e[f]);
+        }
     }
     if (in) return 1;
+    /* the largest kept in registers: an index into s and e would put them in local memory */
     int b = 0;
+    float sb = s[0], eb = e[0];
 #pragma unroll
     for (int f = 1; f < 4; ++f)
-        if (s[f] > s[b]) b = f;
-    if (!(s[b] > e[b])) return 0;
+        if (s[f] > sb) {
+            b = f;
+            sb = s[f];
+            eb = e[f];
+        }
+    if (!(sb > eb)) return 0;
 #pragma unroll
     for (int f = 0; f < 4; ++f)
-        if (f != b && !(s[b] - s[f] > e[b] + e[f])) return 0;
+        if (f != b && !(sb - s[f] > eb + e[f])) return 0;
     fb = b;
     return 2;
 }
@@ -146,6 +162,8 @@ __device__ __forceinline__ int32_t tet_walk(const TetMeshK& m, int32_t t, const 
                      fabs(x[2]) <= (double)m.xmax;
     for (int it = 0; it <= hop_limit; ++it) {
         int fb = 0;
+        /* all four neighbours beside the planes: a hop then waits for one load, not two */
+        const int4 nbr = __ldg(reinterpret_cast<const int4*>(m.nbr) + t);
         const int r = pre ? tet_step32(m, t, x32, fb) : 0;
         if (r == 1) {
             status = TWALK_OK;
@@ -163,7 +181,7 @@ __device__ __forceinline__ int32_t tet_walk(const TetMeshK& m, int32_t t, const 
                 return t;
             }
         }
-        const int32_t nb = __ldg(m.nbr + 4 * (int64_t)t + fb);
+        const int32_t nb = fb == 0 ? nbr.x : (fb == 1 ? nbr.y : (fb == 2 ? nbr.z : nbr.w));
         if (nb < 0) {
             status = TWALK_EXIT;
             return t;
@@ -390,8 +408,15 @@ __global__ void __launch_bounds__(256, TetMinBlocks<V>::value) k_step_tet(const 
 /* the tet step of one cloud on the shared-memory ring                                  */
 /* ------------------------------------------------------------------------------------ */
 
-/* 992-parcel tiles, 31 consumer warps with one slice each (32 warps at 64 registers: the
- * walk's chains of dependent gathers need many warps in flight) */
+/* 992-parcel tiles, 31 consumer warps with one slice each (32 warps at 64 registers).  What
+ * bounds the step are the walk's chains of dependent gathers (owning tet's U and planes ->
+ * neighbour -> its planes), which need many warps in flight and few requests per look: 2e7
+ * parcels on 5.3e6 tets 720 us per launch; planes in 32-byte loads 705; nothing of a look in
+ * local memory 627 (23 consumer warps 756, 27 679); neighbours loaded with the planes 609;
+ * the first planes prefetched 599.  Without the walk it takes 341 us, without the deposits' adds
+ * 75 us less.  Packing the unfinished walks of several slices into full warps was slower (768 at
+ * the same warps, 833 with two slices per warp), and so were prefetches for the next tile
+ * (639). */
 using TetShape = RingShape<992, 31>;
 
 /* The consumer work of the tet ring: each warp's slices of 32 parcels through
@@ -424,6 +449,8 @@ struct TetRing {
                             ring_ld<GLOBAL>(r.w + j)};
                 const V d = ring_ld<GLOBAL>(r.d + j) * a.phys.dscale;
                 int32_t cell = ring_ld<GLOBAL>(r.cell + j);
+                /* the walk's first planes, alongside the cell-velocity gather */
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(a.mesh.planes32 + 4 * (int64_t)cell));
                 bool lost = false;
                 tet_parcel<V, DEP>(a, nsub, pos, vel, d, cell, acc, src, qp, amax, ovf, lost,
                                    key, dep, count_hops);
