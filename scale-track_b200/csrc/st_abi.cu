@@ -128,6 +128,7 @@ struct st_handle {
     size_t psz = 4, vsz = 4;
     void* dU = nullptr;
     double* dsrc = nullptr;
+    uint32_t* dnonzero = nullptr;  /* which parts of dsrc are not zero (launch_finalize) */
     unsigned long long* dacc = nullptr;
     CloudCtl* dctl = nullptr;
     unsigned int* dcounter = nullptr;
@@ -482,13 +483,14 @@ int do_sort_all(st_handle* h)
 }
 
 /* Programmatic dependent launch of the step's kernels: outside graph capture (a captured graph
- * keeps plain edges) and profiling (its events stand between the kernels).  It hides launch gaps of a few microseconds (1e4 parcels on 20^3
- * cells: 13.0 -> 9.5 us per step, 1e5 on 32^3: 15.0 -> 12.3 us), so only handles with small
- * accumulators use it: with large ones the waiting conversion takes SMs from other handles'
- * steps (64 sources of 64^3 cells, three handles in turn: 1526 against 1358 us per step). */
+ * keeps plain edges) and profiling (its events stand between the kernels).  It hides launch
+ * gaps of a few microseconds (1e4 parcels on 20^3 cells: 13.0 -> 9.5 us per step, 1e5 on 32^3:
+ * 15.0 -> 12.3 us), so only handles with accumulators of at most 64 MB use it: with large ones
+ * the waiting conversion takes SMs from other handles' steps (64 sources of 64^3 cells, 403 MB,
+ * three handles in turn: 1526 against 1386 us per step). */
 bool use_pdl(const st_handle* h)
 {
-    return (size_t)h->stride * h->p.n_clouds * h->limbs * 8 <= FINALIZE_CLEAR_BYTES &&
+    return (size_t)h->stride * h->p.n_clouds * h->limbs * 8 <= (size_t)64 << 20 &&
            !h->capturing && !h->prof;
 }
 
@@ -569,7 +571,7 @@ int step_phases(st_handle* h, double dt, int phase, bool empty, L&& launch, S&& 
         h->last_dt = dt;
         if (!det) {
             ProfScope ps(h, ST_KERNEL_OTHER);
-            CK(launch_zero_f64(h->dsrc, (int64_t)nc * h->stride, h->stream));
+            CK(launch_zero_f64(h->dsrc, (int64_t)nc * h->stride, h->stream, use_pdl(h)));
             h->launches += 1;
         }
         if (!empty) {
@@ -592,8 +594,8 @@ int step_phases(st_handle* h, double dt, int phase, bool empty, L&& launch, S&& 
         CK(cudaStreamWaitEvent(h->fin_stream, h->ev_step[p], 0));
         {
             ProfScope ps(h, ST_KERNEL_FINALIZE, h->fin_stream);
-            CK(launch_finalize(h->limbs, acc_ovl, h->dsrc, h->dsrc32, h->dctl, Lf, h->dcounter,
-                               nc, h->stride, finalize_grid(h), h->fin_stream, false));
+            CK(launch_finalize(h->limbs, acc_ovl, h->dsrc, h->dsrc32, h->dnonzero, h->dctl, Lf,
+                               h->dcounter, nc, h->stride, finalize_grid(h), h->fin_stream, false));
         }
         CK(cudaEventRecord(h->ev_fin[p], h->fin_stream));
         h->fin_pending[p] = true;
@@ -603,8 +605,8 @@ int step_phases(st_handle* h, double dt, int phase, bool empty, L&& launch, S&& 
         if (phase == PH_FINISH) CK(launch_ctl_exponents(h->dctl, h->dexp, nc, true, h->stream));
         {
             ProfScope ps(h, ST_KERNEL_FINALIZE);
-            CK(launch_finalize(h->limbs, h->dacc, h->dsrc, h->dsrc32, h->dctl, nullptr,
-                               h->dcounter, nc, h->stride, finalize_grid(h), h->stream,
+            CK(launch_finalize(h->limbs, h->dacc, h->dsrc, h->dsrc32, h->dnonzero, h->dctl,
+                               nullptr, h->dcounter, nc, h->stride, finalize_grid(h), h->stream,
                                use_pdl(h)));
             h->launches += 1;
         }
@@ -1487,9 +1489,11 @@ static int create_impl(const st_params* p, const st_mesh_desc* m, int64_t ncells
     h->own_stream = true;
     const size_t ncomp = (size_t)ncells * 3;
     const size_t cells_total = (size_t)h->stride * p->n_clouds;
+    const size_t nz_bytes = (size_t)((h->stride + 127) / 128) * p->n_clouds * sizeof(uint32_t);
     if ((e = cudaMalloc(&h->dU, ncomp * h->vsz)) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dsrc, cells_total * sizeof(double))) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dacc, cells_total * h->limbs * 8)) != cudaSuccess ||
+        (e = cudaMalloc((void**)&h->dnonzero, nz_bytes)) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dctl, sizeof(CloudCtl) * p->n_clouds)) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dcounter, sizeof(unsigned int))) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dcount, sizeof(unsigned long long))) != cudaSuccess ||
@@ -1500,6 +1504,7 @@ static int create_impl(const st_params* p, const st_mesh_desc* m, int64_t ncells
     if ((e = cudaMemsetAsync(h->dU, 0, ncomp * h->vsz, h->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(h->dsrc, 0, cells_total * sizeof(double), h->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(h->dacc, 0, cells_total * h->limbs * 8, h->stream)) != cudaSuccess ||
+        (e = cudaMemsetAsync(h->dnonzero, 0, nz_bytes, h->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(h->dcounter, 0, sizeof(unsigned int), h->stream)) != cudaSuccess)
         return bail(fail(ST_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e)));
     {
@@ -1689,7 +1694,7 @@ int st_destroy(st_handle* h)
     if (h->graph) cudaGraphDestroy(h->graph);
     void* arrs[] = {h->dU, h->dsrc, h->dacc, h->dctl, h->dcounter, h->dcount, h->dclouds,
                     h->dstage, h->adj.mem, h->dclouds2, h->d_verts, h->d_tets, h->d_planes, h->d_planes32, h->d_nbr,
-                    h->d_hops, h->dbins, h->doffs, h->dscan, h->dexp, h->dacc2, h->dLfin};
+                    h->d_hops, h->dbins, h->doffs, h->dscan, h->dexp, h->dacc2, h->dLfin, h->dnonzero};
     for (void* p : arrs)
         if (p) cudaFree(p);
     for (auto& r : h->recs) {

@@ -304,19 +304,20 @@ cudaError_t ring_prepare();
 template <class P, class V>
 bool ring_eligible(const StepArgs<P, V>& a, int dep);
 
-constexpr size_t FINALIZE_CLEAR_BYTES = (size_t)64 << 20;   /* launch_finalize */
 /* Fixed point -> FP64 source [nclouds][stride] (and, when src32 is not null, its FP32
- * rounding in the same layout), next scale per cloud. */
+ * rounding in the same layout), accumulators cleared, next scale per cloud.  nonzero: one bit
+ * per four components of src, [nclouds][ceil(stride / 128)] words, zero with src. */
 cudaError_t launch_finalize(int limbs, unsigned long long* acc, double* src, float* src32,
-                            CloudCtl* ctl, const int32_t* Lsrc, unsigned int* counter,
-                            int nclouds, int64_t stride, int grid_x, cudaStream_t s, bool pdl);
+                            uint32_t* nonzero, CloudCtl* ctl, const int32_t* Lsrc,
+                            unsigned int* counter, int nclouds, int64_t stride, int grid_x,
+                            cudaStream_t s, bool pdl);
 /* Scale of the step just run -> Lfin, next scale from its largest deposit (overlapped
  * finalize: the finalize then reads Lfin). */
 cudaError_t launch_next_scale(CloudCtl* ctl, int32_t* Lfin, int nclouds, cudaStream_t s);
 cudaError_t launch_set_scale(CloudCtl* ctl, int nclouds, cudaStream_t s);
 cudaError_t launch_ctl_exponents(CloudCtl* ctl, int32_t* e, int nclouds, bool to_ctl,
                                  cudaStream_t s);
-cudaError_t launch_zero_f64(double* p, int64_t n, cudaStream_t s);
+cudaError_t launch_zero_f64(double* p, int64_t n, cudaStream_t s, bool pdl);
 cudaError_t launch_f64_to_f32(const double* in, float* out, int64_t n, cudaStream_t s);
 cudaError_t launch_f32_to_f64(const float* in, double* out, int64_t n, cudaStream_t s);
 template <class P, class V>

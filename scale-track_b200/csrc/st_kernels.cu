@@ -297,12 +297,6 @@ __device__ __forceinline__ void ld32(const unsigned long long* p, unsigned long 
                  : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
                  : "l"(__cvta_generic_to_global(p)));
 }
-__device__ __forceinline__ void ld32_stream(const unsigned long long* p, unsigned long long v[4])
-{
-    asm volatile("ld.global.cs.v4.u64 {%0, %1, %2, %3}, [%4];"
-                 : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
-                 : "l"(__cvta_generic_to_global(p)));
-}
 __device__ __forceinline__ void st32(unsigned long long* p, unsigned long long v)
 {
     asm volatile("st.global.v4.u64 [%0], {%1, %1, %1, %1};" ::"l"(__cvta_generic_to_global(p)),
@@ -317,36 +311,53 @@ __device__ __forceinline__ void st32_stream(double* p, const double v[4])
                  : "memory");
 }
 
-template <int LIMBS, bool CLEAR>
+/* What bounds it is traffic: the accumulator read, the source written, the accumulator cleared
+ * for the step after.  Both writes are left out where nothing is there to write: a group of four
+ * components without deposits is not cleared, and its source is not written again while it is
+ * zero already, which `nonzero` (one bit per group, from the last conversion) remembers.  With
+ * small clouds on a shared mesh most groups are like that: 64 sources of 64^3 cells (403 MB
+ * each of accumulators and sources) 171 us and a memset of 75 us, 207 us with the clearing here,
+ * 183 us with the source's zeros left out too. */
+template <int LIMBS>
 __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict__ acc,
                                                   double* __restrict__ src,
-                                                  float* __restrict__ src32, CloudCtl* ctl,
+                                                  float* __restrict__ src32,
+                                                  uint32_t* __restrict__ nonzero, CloudCtl* ctl,
                                                   const int32_t* __restrict__ Lsrc,
                                                   unsigned int* counter, int nclouds,
                                                   int64_t stride)
 {
+    grid_dep_launch();
+    grid_dep_wait();
     /* stride: per-cloud component count, a multiple of 4 (padding stays zero).  Lsrc: the
      * scale of each cloud when the next scale was already set by k_next_scale (overlapped
      * finalize), else null. */
-    grid_dep_launch();
-    grid_dep_wait();
     const int c = blockIdx.y;
+    const int lane = threadIdx.x & 31;
     const int L = Lsrc ? Lsrc[c] : ctl[c].L;
     unsigned long long* const a = acc + (int64_t)c * stride * LIMBS;
     double* const s = src + (int64_t)c * stride;
     float4* const s32 = src32 ? reinterpret_cast<float4*>(src32 + (int64_t)c * stride) : nullptr;
     const int64_t ngroups = stride / 4;
-    const int64_t gstride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += gstride) {
-        unsigned long long q[4 * LIMBS];
+    const int64_t words = (ngroups + 31) / 32;
+    const int64_t wstride = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    /* a warp takes 32 consecutive groups, one word of `nonzero` */
+    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words;
+         w += wstride) {
+        const int64_t g = 32 * w + lane;
+        const bool valid = g < ngroups;
+        const uint32_t was = nonzero[c * words + w];
+        unsigned long long q[4 * LIMBS] = {};
         unsigned long long any = 0;
+        if (valid) {
 #pragma unroll
-        for (int l = 0; l < LIMBS; ++l) {
-            if (CLEAR) ld32(a + 4 * (LIMBS * g + l), q + 4 * l);
-            else ld32_stream(a + 4 * (LIMBS * g + l), q + 4 * l);
+            for (int l = 0; l < LIMBS; ++l) ld32(a + 4 * (LIMBS * g + l), q + 4 * l);
         }
 #pragma unroll
         for (int k = 0; k < 4 * LIMBS; ++k) any |= q[k];
+        const uint32_t now = __ballot_sync(FULL_MASK, any != 0);
+        if (lane == 0 && now != was) nonzero[c * words + w] = now;
+        if (!valid) continue;
         double o[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -362,9 +373,8 @@ __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict
             }
             o[k] = ldexp2(v, L);
         }
-        st32_stream(s + 4 * g, o);
-        /* cleared for the step after, where there is anything to clear */
-        if (CLEAR && any) {
+        if (any || (was >> lane & 1u)) st32_stream(s + 4 * g, o);
+        if (any) {
 #pragma unroll
             for (int l = 0; l < LIMBS; ++l) st32(a + 4 * (LIMBS * g + l), 0ULL);
         }
@@ -391,25 +401,15 @@ __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict
     }
 }
 
-/* Accumulators up to FINALIZE_CLEAR_BYTES are cleared by the conversion as it reads them, which saves the
- * memset's launch behind every step (1e4 parcels on 20^3 cells: 16.2 -> 13.0 us per step, 4e6
- * on 64^3: 92.8 -> 88.6 us); 128^3 cells (50 MB) are even.  Larger ones exceed the L2 together
- * with the source and U: there zeros written between the reads are slower than a memset of
- * its own (64 sources of 64^3 cells, 403 MB: 1462 against 1358 us per step). */
 cudaError_t launch_finalize(int limbs, unsigned long long* acc, double* src, float* src32,
-                            CloudCtl* ctl, const int32_t* Lsrc, unsigned int* counter,
-                            int nclouds, int64_t stride, int grid_x, cudaStream_t s, bool pdl)
+                            uint32_t* nonzero, CloudCtl* ctl, const int32_t* Lsrc,
+                            unsigned int* counter, int nclouds, int64_t stride, int grid_x,
+                            cudaStream_t s, bool pdl)
 {
     if (stride % 4) return cudaErrorInvalidValue;
-    dim3 grid(grid_x, nclouds);
-    const size_t bytes = (size_t)stride * nclouds * limbs * 8;
-    const bool clear = bytes <= FINALIZE_CLEAR_BYTES;
-    const auto k = limbs == 1 ? (clear ? k_finalize<1, true> : k_finalize<1, false>)
-                              : (clear ? k_finalize<2, true> : k_finalize<2, false>);
-    const cudaError_t e = launch_kernel(pdl, k, grid, dim3(256), 0, s, acc, src, src32, ctl, Lsrc,
-                                        counter, nclouds, stride);
-    if (e != cudaSuccess || clear) return e;
-    return cudaMemsetAsync(acc, 0, bytes, s);
+    return launch_kernel(pdl, limbs == 1 ? k_finalize<1> : k_finalize<2>, dim3(grid_x, nclouds),
+                         dim3(256), 0, s, acc, src, src32, nonzero, ctl, Lsrc, counter, nclouds,
+                         stride);
 }
 
 /* The scale bookkeeping of k_finalize on its own, for an overlapped finalize: keeps each
@@ -467,21 +467,21 @@ cudaError_t launch_set_scale(CloudCtl* ctl, int nclouds, cudaStream_t s)
     return cudaGetLastError();
 }
 
-__global__ void k_zero_f64(double* p, int64_t n)
+__global__ void __launch_bounds__(256) k_zero_f64(double* p, int64_t n)
 {
-    /* n is a multiple of 2 and p 16-byte aligned (padded per-cloud strides) */
-    double2* q = reinterpret_cast<double2*>(p);
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n / 2;
+    grid_dep_launch();
+    grid_dep_wait();
+    /* n is a multiple of 4 and p 32-byte aligned (padded per-cloud strides) */
+    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n / 4;
          j += (int64_t)gridDim.x * blockDim.x)
-        q[j] = make_double2(0.0, 0.0);
+        st32(reinterpret_cast<unsigned long long*>(p) + 4 * j, 0ULL);
 }
 
-cudaError_t launch_zero_f64(double* p, int64_t n, cudaStream_t s)
+cudaError_t launch_zero_f64(double* p, int64_t n, cudaStream_t s, bool pdl)
 {
-    int grid = (int)((n + 255) / 256 < 148 * 8 ? (n + 255) / 256 : 148 * 8);
-    if (grid < 1) grid = 1;
-    k_zero_f64<<<grid, 256, 0, s>>>(p, n);
-    return cudaGetLastError();
+    const int64_t g = (n / 4 + 255) / 256;
+    const int grid = (int)(g < 1 ? 1 : (g < 148 * 8 ? g : 148 * 8));
+    return launch_kernel(pdl, k_zero_f64, dim3(grid), dim3(256), 0, s, p, n);
 }
 
 __global__ void k_f64_to_f32(const double* __restrict__ in, float* __restrict__ out, int64_t n)

@@ -133,3 +133,46 @@ def test_noalloc_calls_in_a_row(npcl):
         if npcl:
             assert np.array_equal(np.stack([t.cpu().numpy() for t in X]), px)
             assert np.array_equal(np.stack([t.cpu().numpy() for t in V]).astype(np.float64), pv)
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("n", [3, 5, 11])
+def test_sources_empty_where_parcels_left(prec, n):
+    """The conversion writes a part of the source only where there is something now or was
+    before: three clouds (one empty, one in a corner, one everywhere) whose parcels are replaced
+    twice, with component counts that leave ragged groups of four and ragged words of 32 groups.
+    Each source, in 8 and 4 bytes, equals that of a handle that never held other parcels."""
+    U = workload.tgv_field(n, U0=2.0, dtype=np.float64 if prec == "fp64" else np.float32)
+    mesh = st.mesh_desc(n, 0.0, workload.L_BOX)
+
+    def prm(nc):
+        return st.params(mu_c=workload.MU_F, rho_c=workload.RHO_F, rho_d=workload.RHO_P,
+                         drag_model="schiller_naumann", precision=prec, n_substeps=1, n_clouds=nc)
+
+    def clouds(rep):
+        out = []
+        for c, npcl in enumerate((0, 40, 700)):
+            xyz, uvw, d = workload.parcels(npcl, 7 * rep + c)
+            if c == 1:
+                xyz = xyz / n if rep % 2 == 0 else workload.L_BOX * (1 - 1e-6) - xyz / n
+            out.append((xyz, uvw, d))
+        return out
+
+    with st.ParcelTracker(prm(3), mesh) as h:
+        h.set_fluid_velocity(U)
+        for rep in range(3):
+            for c, p in enumerate(clouds(rep)):
+                h.set_parcels(*p, cloud=c)
+            for _ in range(2):
+                h.step(workload.DT)
+            for c, p in enumerate(clouds(rep)):
+                with st.ParcelTracker(prm(1), mesh) as f:
+                    f.set_fluid_velocity(U)
+                    f.set_parcels(*p)
+                    for _ in range(2):
+                        f.step(workload.DT)
+                    ref = f.get_source()
+                got = h.get_source(cloud=c)
+                assert np.array_equal(got, ref)
+                assert np.array_equal(h.get_source(cloud=c, dtype=np.float32), ref.astype(np.float32))
+                assert (np.abs(ref).max() > 0) == (c > 0)
