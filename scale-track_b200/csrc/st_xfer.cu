@@ -12,7 +12,7 @@
  * 162 -> 30 ms, an adjoint pass with 124 MB in and out 18.6 -> 10.7 ms, a 64^3 coupled step
  * with double fields 0.78 -> 0.75 ms.
  *
- * The staging buffers belong to the process: XFER_THREADS pinned pieces (16 MB), made by the
+ * The staging buffers belong to the process: XFER_THREADS pinned pieces (24 MB), made by the
  * first copy of XFER_MIN bytes or more and freed with the last handle.  One copy uses them at a
  * time; a copy that finds them taken (another host thread's), or cannot have them, and copies
  * to pinned memory or below XFER_MIN, go through plain cudaMemcpyAsync.
@@ -31,10 +31,11 @@ namespace st {
 namespace {
 
 /* 2 MB pieces, 1 MB below 16 MB in all (three 2 MB pieces would leave threads without one):
- * the read-back below 3.03 -> 2.85 ms; pieces of 256 KB 3.5 ms. */
+ * the read-back above 3.03 -> 2.85 ms; pieces of 256 KB 3.5 ms.  Twelve threads against eight:
+ * 50 MB into fresh pages 3.43 -> 3.02 ms, sixteen 3.74 ms. */
 constexpr size_t XFER_PIECE = (size_t)2 << 20;
 constexpr size_t XFER_MIN = (size_t)2 << 20;
-constexpr int XFER_THREADS = 8;
+constexpr int XFER_THREADS = 12;
 
 std::mutex g_users_mu;
 int g_users = 0;             /* live handles */
