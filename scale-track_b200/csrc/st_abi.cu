@@ -128,7 +128,6 @@ struct st_handle {
     size_t psz = 4, vsz = 4;
     void* dU = nullptr;
     double* dsrc = nullptr;
-    uint32_t* dnonzero = nullptr;  /* which parts of dsrc are not zero (launch_finalize) */
     unsigned long long* dacc = nullptr;
     CloudCtl* dctl = nullptr;
     unsigned int* dcounter = nullptr;
@@ -485,12 +484,19 @@ int do_sort_all(st_handle* h)
 /* Programmatic dependent launch of the step's kernels: outside graph capture (a captured graph
  * keeps plain edges) and profiling (its events stand between the kernels).  It hides launch
  * gaps of a few microseconds (1e4 parcels on 20^3 cells: 13.0 -> 9.5 us per step, 1e5 on 32^3:
- * 15.0 -> 12.3 us), so only handles with accumulators of at most 64 MB use it: with large ones
- * the waiting conversion takes SMs from other handles' steps (64 sources of 64^3 cells, 403 MB,
- * three handles in turn: 1526 against 1386 us per step). */
+ * 15.0 -> 12.3 us), so only small steps use it: accumulators of at most 8 MB and 5e5 parcels.
+ * Beyond, the blocks that wait take SMs from other handles' steps (three handles in turn, with
+ * and without: 14 clouds, 15 MB, two steps 41 and 35 us; 20 FP64 clouds, 23 MB, 121 and 108; one
+ * cloud of 4e6 parcels, 4 MB, two times ten substeps 650 and 597; 2.5e5 parcels, 0.4 MB, 64 and
+ * 68). */
+constexpr size_t PDL_BYTES = (size_t)8 << 20;
+constexpr int64_t PDL_PARCELS = 500000;
+
+size_t acc_bytes(const st_handle* h) { return (size_t)h->stride * h->p.n_clouds * h->limbs * 8; }
+
 bool use_pdl(const st_handle* h)
 {
-    return (size_t)h->stride * h->p.n_clouds * h->limbs * 8 <= (size_t)64 << 20 &&
+    return acc_bytes(h) <= PDL_BYTES && h->total_tiles <= PDL_PARCELS / WARP_TILE &&
            !h->capturing && !h->prof;
 }
 
@@ -503,6 +509,12 @@ bool use_pdl(const st_handle* h)
  *   hex, FP32 and mixed:  1e4 15.9 / 9.5   1e5 14.6 / 12.3   1.5e6 41.1 / 41.0   4e6 84.5 / 92.6
  *   hex, FP64:   1e5 17.7 / 15.0   4e5 25.2 / 24.9   5e5 30.1 / 32.1   4e6 141 / 151
  *   hex, mixed, ten substeps:  1e6 118 / 99   4e6 386 / 333   1e7 987 / 859
+ * On larger meshes the conversion weighs more, and the ring's overlapped one pays earlier (two
+ * steps, three handles in turn):
+ *   mixed, 76^3:  1e5 29.8 / 40.7   1e6 65.8 / 76.9;  128^3:  1e5 65.5 / 79.5   1e6 136 / 149
+ *   mixed, 90^3:  2e4 32.5 / 28.2;  FP64, 60^3:  1e5 30.9 / 35.5;  100^3:  1e5 61.8 / 74.7
+ *   mixed, 60^3:  1e5 28.1 / 24.3   3e5 28.1 / 29.6   7e5 46.3 / 49.6
+ *   mixed, 48^3:  3e5 26.2 / 23.4   1.3e6 63.5 / 61.8;  FP64, 48^3:  3e5 35.1 / 33.4
  *   tet, mixed:  2e5 22.0 / 20.4   4e5 27.1 / 27.6   1e6 43.6 / 46.2; three substeps: 1e6 73 / 78
  *   tet, FP64:   4e5 33.6 / 35.3   1e6 75.2 / 79.4   2e6 123 / 131
  * A wait limit set by the caller is about the ring's waits: the ring then runs at any size. */
@@ -512,7 +524,10 @@ bool use_ring(const st_handle* h, int64_t n)
     if (h->wait_cycles != 0) return true;
     const bool fp64 = h->p.precision == ST_PREC_FP64;
     if (h->tet) return n >= 300000;
-    return h->p.n_substeps == 1 && n >= (fp64 ? 450000 : 1500000);
+    if (h->p.n_substeps != 1) return false;
+    if (acc_bytes(h) > PDL_BYTES && n >= 50000) return true;
+    if (h->stride >= 3 * 200000 && n >= 250000) return true;
+    return n >= (fp64 ? 450000 : 1500000);
 }
 
 /* Phases of one step.  PH_ALL is st_step.  A sharded step (one handle per rank, parcels
@@ -594,8 +609,8 @@ int step_phases(st_handle* h, double dt, int phase, bool empty, L&& launch, S&& 
         CK(cudaStreamWaitEvent(h->fin_stream, h->ev_step[p], 0));
         {
             ProfScope ps(h, ST_KERNEL_FINALIZE, h->fin_stream);
-            CK(launch_finalize(h->limbs, acc_ovl, h->dsrc, h->dsrc32, h->dnonzero, h->dctl, Lf,
-                               h->dcounter, nc, h->stride, finalize_grid(h), h->fin_stream, false));
+            CK(launch_finalize(h->limbs, acc_ovl, h->dsrc, h->dsrc32, h->dctl, Lf, h->dcounter,
+                               nc, h->stride, finalize_grid(h), h->fin_stream, false));
         }
         CK(cudaEventRecord(h->ev_fin[p], h->fin_stream));
         h->fin_pending[p] = true;
@@ -605,8 +620,8 @@ int step_phases(st_handle* h, double dt, int phase, bool empty, L&& launch, S&& 
         if (phase == PH_FINISH) CK(launch_ctl_exponents(h->dctl, h->dexp, nc, true, h->stream));
         {
             ProfScope ps(h, ST_KERNEL_FINALIZE);
-            CK(launch_finalize(h->limbs, h->dacc, h->dsrc, h->dsrc32, h->dnonzero, h->dctl,
-                               nullptr, h->dcounter, nc, h->stride, finalize_grid(h), h->stream,
+            CK(launch_finalize(h->limbs, h->dacc, h->dsrc, h->dsrc32, h->dctl, nullptr,
+                               h->dcounter, nc, h->stride, finalize_grid(h), h->stream,
                                use_pdl(h)));
             h->launches += 1;
         }
@@ -1489,11 +1504,9 @@ static int create_impl(const st_params* p, const st_mesh_desc* m, int64_t ncells
     h->own_stream = true;
     const size_t ncomp = (size_t)ncells * 3;
     const size_t cells_total = (size_t)h->stride * p->n_clouds;
-    const size_t nz_bytes = (size_t)((h->stride + 127) / 128) * p->n_clouds * sizeof(uint32_t);
     if ((e = cudaMalloc(&h->dU, ncomp * h->vsz)) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dsrc, cells_total * sizeof(double))) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dacc, cells_total * h->limbs * 8)) != cudaSuccess ||
-        (e = cudaMalloc((void**)&h->dnonzero, nz_bytes)) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dctl, sizeof(CloudCtl) * p->n_clouds)) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dcounter, sizeof(unsigned int))) != cudaSuccess ||
         (e = cudaMalloc((void**)&h->dcount, sizeof(unsigned long long))) != cudaSuccess ||
@@ -1504,7 +1517,6 @@ static int create_impl(const st_params* p, const st_mesh_desc* m, int64_t ncells
     if ((e = cudaMemsetAsync(h->dU, 0, ncomp * h->vsz, h->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(h->dsrc, 0, cells_total * sizeof(double), h->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(h->dacc, 0, cells_total * h->limbs * 8, h->stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(h->dnonzero, 0, nz_bytes, h->stream)) != cudaSuccess ||
         (e = cudaMemsetAsync(h->dcounter, 0, sizeof(unsigned int), h->stream)) != cudaSuccess)
         return bail(fail(ST_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e)));
     {
@@ -1694,7 +1706,7 @@ int st_destroy(st_handle* h)
     if (h->graph) cudaGraphDestroy(h->graph);
     void* arrs[] = {h->dU, h->dsrc, h->dacc, h->dctl, h->dcounter, h->dcount, h->dclouds,
                     h->dstage, h->adj.mem, h->dclouds2, h->d_verts, h->d_tets, h->d_planes, h->d_planes32, h->d_nbr,
-                    h->d_hops, h->dbins, h->doffs, h->dscan, h->dexp, h->dacc2, h->dLfin, h->dnonzero};
+                    h->d_hops, h->dbins, h->doffs, h->dscan, h->dexp, h->dacc2, h->dLfin};
     for (void* p : arrs)
         if (p) cudaFree(p);
     for (auto& r : h->recs) {

@@ -29,7 +29,7 @@
  * a step is the start cell of the next unless the parcel bounced.  The records are held per
  * resident block, not per parcel, so that they stay in the L2 between writing and reading.
  * 1e6 parcels on 128^3 cells, 200 steps, checkpoints every 20, mixed precision: forward
- * 3.89 -> 1.78 ms (2.96 ms with every step's deposits going to memory), reverse 3.88 -> 2.78 ms
+ * 3.89 -> 1.75 ms (2.96 ms with every step's deposits going to memory), reverse 3.88 -> 2.63 ms
  * (records per parcel in HBM, power and cell velocity formed again in the reverse step before).
  */
 #include <cstdint>

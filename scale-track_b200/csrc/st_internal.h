@@ -305,12 +305,10 @@ template <class P, class V>
 bool ring_eligible(const StepArgs<P, V>& a, int dep);
 
 /* Fixed point -> FP64 source [nclouds][stride] (and, when src32 is not null, its FP32
- * rounding in the same layout), accumulators cleared, next scale per cloud.  nonzero: one bit
- * per four components of src, [nclouds][ceil(stride / 128)] words, zero with src. */
+ * rounding in the same layout), accumulators cleared, next scale per cloud. */
 cudaError_t launch_finalize(int limbs, unsigned long long* acc, double* src, float* src32,
-                            uint32_t* nonzero, CloudCtl* ctl, const int32_t* Lsrc,
-                            unsigned int* counter, int nclouds, int64_t stride, int grid_x,
-                            cudaStream_t s, bool pdl);
+                            CloudCtl* ctl, const int32_t* Lsrc, unsigned int* counter,
+                            int nclouds, int64_t stride, int grid_x, cudaStream_t s, bool pdl);
 /* Scale of the step just run -> Lfin, next scale from its largest deposit (overlapped
  * finalize: the finalize then reads Lfin). */
 cudaError_t launch_next_scale(CloudCtl* ctl, int32_t* Lfin, int nclouds, cudaStream_t s);

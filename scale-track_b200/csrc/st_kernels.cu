@@ -312,17 +312,14 @@ __device__ __forceinline__ void st32_stream(double* p, const double v[4])
 }
 
 /* What bounds it is traffic: the accumulator read, the source written, the accumulator cleared
- * for the step after.  Both writes are left out where nothing is there to write: a group of four
- * components without deposits is not cleared, and its source is not written again while it is
- * zero already, which `nonzero` (one bit per group, from the last conversion) remembers.  With
- * small clouds on a shared mesh most groups are like that: 64 sources of 64^3 cells (403 MB
- * each of accumulators and sources) 171 us and a memset of 75 us, 207 us with the clearing here,
- * 183 us with the source's zeros left out too. */
-template <int LIMBS>
+ * for the step after.  CLEAR: the clearing here, of the groups of four components that hold
+ * something (few with small clouds on a shared mesh: 64 sources of 64^3 cells, 403 MB each of
+ * accumulators and sources, 207 us; 171 us and a memset of 75 us without).  The source is
+ * written whole, zeros included: callers hold its device pointer. */
+template <int LIMBS, bool CLEAR>
 __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict__ acc,
                                                   double* __restrict__ src,
-                                                  float* __restrict__ src32,
-                                                  uint32_t* __restrict__ nonzero, CloudCtl* ctl,
+                                                  float* __restrict__ src32, CloudCtl* ctl,
                                                   const int32_t* __restrict__ Lsrc,
                                                   unsigned int* counter, int nclouds,
                                                   int64_t stride)
@@ -333,31 +330,31 @@ __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict
      * scale of each cloud when the next scale was already set by k_next_scale (overlapped
      * finalize), else null. */
     const int c = blockIdx.y;
-    const int lane = threadIdx.x & 31;
     const int L = Lsrc ? Lsrc[c] : ctl[c].L;
     unsigned long long* const a = acc + (int64_t)c * stride * LIMBS;
     double* const s = src + (int64_t)c * stride;
     float4* const s32 = src32 ? reinterpret_cast<float4*>(src32 + (int64_t)c * stride) : nullptr;
     const int64_t ngroups = stride / 4;
-    const int64_t words = (ngroups + 31) / 32;
-    const int64_t wstride = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    /* a warp takes 32 consecutive groups, one word of `nonzero` */
-    for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words;
-         w += wstride) {
-        const int64_t g = 32 * w + lane;
-        const bool valid = g < ngroups;
-        const uint32_t was = nonzero[c * words + w];
-        unsigned long long q[4 * LIMBS] = {};
+    const int64_t gstride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += gstride) {
+        unsigned long long q[4 * LIMBS];
         unsigned long long any = 0;
-        if (valid) {
 #pragma unroll
-            for (int l = 0; l < LIMBS; ++l) ld32(a + 4 * (LIMBS * g + l), q + 4 * l);
+        for (int l = 0; l < LIMBS; ++l) {
+            const unsigned long long* const p = a + 4 * (LIMBS * g + l);
+            if (CLEAR) {
+                ld32(p, q + 4 * l);
+            } else {
+                const ulonglong2 q0 = __ldcs(reinterpret_cast<const ulonglong2*>(p));
+                const ulonglong2 q1 = __ldcs(reinterpret_cast<const ulonglong2*>(p) + 1);
+                q[4 * l] = q0.x;
+                q[4 * l + 1] = q0.y;
+                q[4 * l + 2] = q1.x;
+                q[4 * l + 3] = q1.y;
+            }
         }
 #pragma unroll
         for (int k = 0; k < 4 * LIMBS; ++k) any |= q[k];
-        const uint32_t now = __ballot_sync(FULL_MASK, any != 0);
-        if (lane == 0 && now != was) nonzero[c * words + w] = now;
-        if (!valid) continue;
         double o[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -373,8 +370,13 @@ __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict
             }
             o[k] = ldexp2(v, L);
         }
-        if (any || (was >> lane & 1u)) st32_stream(s + 4 * g, o);
-        if (any) {
+        if (CLEAR) {
+            st32_stream(s + 4 * g, o);
+        } else {
+            __stcs(reinterpret_cast<double2*>(s + 4 * g), make_double2(o[0], o[1]));
+            __stcs(reinterpret_cast<double2*>(s + 4 * g) + 1, make_double2(o[2], o[3]));
+        }
+        if (CLEAR && any) {
 #pragma unroll
             for (int l = 0; l < LIMBS; ++l) st32(a + 4 * (LIMBS * g + l), 0ULL);
         }
@@ -401,15 +403,25 @@ __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict
     }
 }
 
+/* Where the accumulators are cleared.  Those of one cloud, small ones, and those far larger than
+ * the L2, by the conversion (15 MB of accumulators, three handles in turn: 35 against 39 us per
+ * pass of two steps; 403 MB: 1207 against 1386 us; one cloud on 1.6e6 tets, 38 MB: 62.6 against
+ * 66 us).  Between, where the accumulators of many clouds fit the L2 but not along with all
+ * else, they are read evict-first and a memset of its own leaves their zeros in the L2 for the
+ * step's adds (33 MB: 145 against 165 us; 36 MB: 84 against 90; 84 MB: 217 against 220). */
 cudaError_t launch_finalize(int limbs, unsigned long long* acc, double* src, float* src32,
-                            uint32_t* nonzero, CloudCtl* ctl, const int32_t* Lsrc,
-                            unsigned int* counter, int nclouds, int64_t stride, int grid_x,
-                            cudaStream_t s, bool pdl)
+                            CloudCtl* ctl, const int32_t* Lsrc, unsigned int* counter,
+                            int nclouds, int64_t stride, int grid_x, cudaStream_t s, bool pdl)
 {
     if (stride % 4) return cudaErrorInvalidValue;
-    return launch_kernel(pdl, limbs == 1 ? k_finalize<1> : k_finalize<2>, dim3(grid_x, nclouds),
-                         dim3(256), 0, s, acc, src, src32, nonzero, ctl, Lsrc, counter, nclouds,
-                         stride);
+    const size_t bytes = (size_t)stride * nclouds * limbs * 8;
+    const bool clear = nclouds == 1 || bytes <= (size_t)24 << 20 || bytes > (size_t)96 << 20;
+    const auto k = limbs == 1 ? (clear ? k_finalize<1, true> : k_finalize<1, false>)
+                              : (clear ? k_finalize<2, true> : k_finalize<2, false>);
+    const cudaError_t e = launch_kernel(pdl && clear, k, dim3(grid_x, nclouds), dim3(256), 0, s,
+                                        acc, src, src32, ctl, Lsrc, counter, nclouds, stride);
+    if (e != cudaSuccess || clear) return e;
+    return cudaMemsetAsync(acc, 0, bytes, s);
 }
 
 /* The scale bookkeeping of k_finalize on its own, for an overlapped finalize: keeps each

@@ -135,13 +135,20 @@ def test_noalloc_calls_in_a_row(npcl):
             assert np.array_equal(np.stack([t.cpu().numpy() for t in V]).astype(np.float64), pv)
 
 
+class _DeviceArray:
+    def __init__(self, ptr, n):
+        self.__cuda_array_interface__ = dict(shape=(n,), typestr="<f8", data=(ptr, False),
+                                             version=2)
+
+
 @pytest.mark.parametrize("prec", ["mixed", "fp64"])
 @pytest.mark.parametrize("n", [3, 5, 11])
 def test_sources_empty_where_parcels_left(prec, n):
-    """The conversion writes a part of the source only where there is something now or was
-    before: three clouds (one empty, one in a corner, one everywhere) whose parcels are replaced
-    twice, with component counts that leave ragged groups of four and ragged words of 32 groups.
-    Each source, in 8 and 4 bytes, equals that of a handle that never held other parcels."""
+    """The conversion clears an accumulator only where something was added, and writes the whole
+    source also over what its holder wrote there: three clouds (one empty, one in a corner, one
+    everywhere) whose parcels are replaced twice, with component counts that leave ragged groups
+    of four.  Each source, in 8 and 4 bytes, equals that of a handle that never held others."""
+    import torch
     U = workload.tgv_field(n, U0=2.0, dtype=np.float64 if prec == "fp64" else np.float32)
     mesh = st.mesh_desc(n, 0.0, workload.L_BOX)
 
@@ -163,8 +170,13 @@ def test_sources_empty_where_parcels_left(prec, n):
         for rep in range(3):
             for c, p in enumerate(clouds(rep)):
                 h.set_parcels(*p, cloud=c)
-            for _ in range(2):
-                h.step(workload.DT)
+            h.step(workload.DT)
+            h.synchronize()
+            for c in range(3):
+                src = _DeviceArray(h.source_device_ptr(c), 3 * n**3)
+                torch.as_tensor(src, device="cuda").fill_(1.5)
+            torch.cuda.synchronize()
+            h.step(workload.DT)
             for c, p in enumerate(clouds(rep)):
                 with st.ParcelTracker(prm(1), mesh) as f:
                     f.set_fluid_velocity(U)
