@@ -268,7 +268,10 @@ void st_set_last_error(const char* msg);
 
 /* Launches a kernel whose launch and block set-up may overlap the end of the kernel before it
  * on the stream (programmatic dependent launch, pdl = true).  The kernel calls
- * grid_dep_wait() before it touches memory. */
+ * grid_dep_wait() before it touches memory, and it reads what a programmatically launched
+ * chain writes (parcels, accumulators, control blocks) by plain or inline-assembly loads only:
+ * its blocks may be resident while the kernels before it still write, and data read through
+ * __ldg or a const __restrict__ pointer must not change while a kernel is resident. */
 template <class... K, class... A>
 cudaError_t launch_kernel(bool pdl, void (*kernel)(K...), dim3 grid, dim3 block, size_t smem,
                           cudaStream_t s, const A&... args)

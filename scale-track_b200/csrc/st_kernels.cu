@@ -320,7 +320,7 @@ template <int LIMBS, bool CLEAR>
 __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict__ acc,
                                                   double* __restrict__ src,
                                                   float* __restrict__ src32, CloudCtl* ctl,
-                                                  const int32_t* __restrict__ Lsrc,
+                                                  const int32_t* Lsrc,
                                                   unsigned int* counter, int nclouds,
                                                   int64_t stride)
 {

@@ -85,10 +85,14 @@ __global__ void k_noalloc_reset(CtlPair* both)
  * What bounds the smallest calls is the chain's latency and the read-back of the control block:
  * 3001 parcels on 12^3 cells took 48.8 us as a memset and five kernels in stream order with the
  * occupancy queried on every call, 32.0 us now (a kernel and a read-back alone: 20 us); 1e6 on
- * 64^3 cells 87.6 -> 78.4 us. */
+ * 64^3 cells 87.6 -> 78.4 us.
+ *
+ * acc: plain loads.  The blocks of this kernel may be resident while the probe still clears the
+ * accumulator and the step adds to it, so it is not read-only for the kernel's lifetime, as
+ * const __restrict__ or __ldg would promise. */
 __global__ void __launch_bounds__(256) k_noalloc_finalize(
-    const unsigned long long* __restrict__ acc, const CtlPair* ctl, CtlPair* next, int H,
-    double* __restrict__ src, int64_t ncomp)
+    const unsigned long long* acc, const CtlPair* ctl, CtlPair* next, int H, double* src,
+    int64_t ncomp)
 {
     grid_dep_wait();
     if (blockIdx.x == 0 && threadIdx.x == 0) reset(next);
