@@ -1189,16 +1189,15 @@ int graph_capture(st_handle* h, int n, double dt, const double* fs)
     return ST_OK;
 }
 
+/* The persistent grid of the per-warp step kernel: SMs x resident blocks of that size. */
 int occupancy_grid(st_handle* h, int block)
 {
-    int nsm = 148;
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device);
-    int occ = h->p.precision == ST_PREC_FP32
-                  ? step_max_active_blocks<float, float>(h->dep, block)
-                  : (h->p.precision == ST_PREC_MIXED
-                         ? step_max_active_blocks<double, float>(h->dep, block)
-                         : step_max_active_blocks<double, double>(h->dep, block));
-    return nsm * (occ < 1 ? 1 : occ);
+    const int nsub = h->p.n_substeps, nc = h->p.n_clouds;
+    const int occ = h->tet ? (h->p.precision == ST_PREC_FP64
+                                  ? step_tet_max_active_blocks<double>(h->dep, block)
+                                  : step_tet_max_active_blocks<float>(h->dep, block))
+                           : DISPATCH(h, step_max_active_blocks, h->dep, block, nsub, nc);
+    return h->nsm * (occ < 1 ? 1 : occ);
 }
 
 }  // namespace
@@ -1594,12 +1593,7 @@ static int create_impl(const st_params* p, const st_mesh_desc* m, int64_t ncells
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
     h->nsm = nsm > 0 ? nsm : 148;
-    int occ = h->tet ? (p->precision == ST_PREC_FP64
-                            ? step_tet_max_active_blocks<double>(h->dep, h->block)
-                            : step_tet_max_active_blocks<float>(h->dep, h->block))
-                     : DISPATCH(h, step_max_active_blocks, h->dep, h->block);
-    if (occ < 1) occ = 1;
-    h->grid = p->grid_blocks > 0 ? p->grid_blocks : nsm * occ;
+    h->grid = p->grid_blocks > 0 ? p->grid_blocks : occupancy_grid(h, h->block);
     if (!h->tet && (e = DISPATCH(h, ring_prepare)) != cudaSuccess)
         return bail(fail(ST_ERR_CUDA, "ring kernel set-up: %s", cudaGetErrorString(e)));
     if (h->tet && (e = (p->precision == ST_PREC_FP64 ? tet_ring_prepare<double>()

@@ -293,8 +293,9 @@ cudaError_t launch_kernel(bool pdl, void (*kernel)(K...), dim3 grid, dim3 block,
 template <class P, class V>
 cudaError_t launch_step(const StepArgs<P, V>& a, int dep, int grid, int block, cudaStream_t s,
                         bool pdl = false);
+/* Resident blocks per SM of the step kernel for a handle of nclouds clouds and nsub substeps. */
 template <class P, class V>
-int step_max_active_blocks(int dep, int block);
+int step_max_active_blocks(int dep, int block, int nsub, int nclouds);
 /* The step of a single cloud as a persistent shared-memory ring (st_ring.cu); deposits
  * DEP_DET1, DEP_DET2 or DEP_ATOMIC.  Every parcel array must be 16-byte aligned. */
 template <class P, class V>

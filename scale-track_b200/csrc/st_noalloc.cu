@@ -51,7 +51,7 @@ constexpr int MAX_DEVICES = 64;
 struct Scratch {
     CtlPair* ctl = nullptr;
     unsigned long long* acc = nullptr;
-    int resident = 0;    /* step blocks that stay resident on the device */
+    int resident[2] = {0, 0};  /* step blocks that stay resident on the device: one substep, several */
     int next = 0;        /* the control set of the next call */
     bool dirty = false;  /* a call failed before its last kernel: both sets need a reset */
 };
@@ -175,8 +175,10 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
             if (e != cudaSuccess || !pc || !pa) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
             int nsm = 148;
             cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-            const int occ = step_max_active_blocks<double, float>(DEP_DET1, 256);
-            g.resident = nsm * (occ < 1 ? 1 : occ);
+            for (int sub = 0; sub < 2; ++sub) {
+                const int occ = step_max_active_blocks<double, float>(DEP_DET1, 256, sub + 1, 1);
+                g.resident[sub] = nsm * (occ < 1 ? 1 : occ);
+            }
             g.ctl = static_cast<CtlPair*>(pc);
             g.acc = static_cast<unsigned long long*>(pa);
         }
@@ -188,6 +190,7 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
     unsigned long long* const acc = sc.acc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int64_t ncomp = ncells * 3;
+    const int64_t resident = sc.resident[p->n_substeps > 1];
 
     const int64_t bound = n * (int64_t)p->n_substeps > 2 ? n * (int64_t)p->n_substeps : 2;
     const int H = 62 - QUANT_GROWTH_BITS - quant_nbits(bound);
@@ -241,7 +244,7 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
         probe.ctl = &ctl->probe;
         probe.clear = acc;
         probe.clear_n = ncomp;
-        e = launch_step<double, float>(probe, DEP_PROBE, (int)std::min<int64_t>(need, sc.resident),
+        e = launch_step<double, float>(probe, DEP_PROBE, (int)std::min(need, resident),
                                        256, s, false);
         if (e != cudaSuccess) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
     }
@@ -249,7 +252,7 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
         const int64_t need = (a.total_tiles + 7) / 8;
         a.probed = &ctl->probe;
         a.H = H;
-        e = launch_step<double, float>(a, DEP_DET1, (int)std::min<int64_t>(need, sc.resident), 256,
+        e = launch_step<double, float>(a, DEP_DET1, (int)std::min(need, resident), 256,
                                        s, true);
         if (e != cudaSuccess) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
     }
