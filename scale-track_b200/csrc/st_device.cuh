@@ -349,8 +349,8 @@ __device__ __forceinline__ T ld_stream(const T* p) { return ld_stream_(p); }
 template <class T>
 __device__ __forceinline__ void st_stream(T* p, T v) { __stcs(p, v); }
 
-/* 8-byte words of shared memory that one warp's deposit_warp needs (its last argument): up to
- * 96 sums and the 32 cells they go to. */
+/* 8-byte words of shared memory, 16-byte aligned, that one warp's deposit_warp needs: up to 96
+ * sums and the 32 cells they go to. */
 template <int DEP, class V>
 constexpr int dep_ws_words = DEP == DEP_ATOMIC                  ? 96 + 16
                              : DEP == DEP_DET1 && sizeof(V) == 4 ? 48 + 16
@@ -363,7 +363,8 @@ constexpr int dep_ws_words = DEP == DEP_ATOMIC                  ? 96 + 16
  * per component sends every value as a request of its own.  The adds were what bound the hex
  * step once parcels have drifted from their sorted order (1e7 parcels on 128^3 cells, mean of
  * a re-sort cycle of 20 steps, conversion in stream order: 209 us per launch, 146 us with the
- * adds left out, 186 us with this hand-over and the longer chunks of scan_steps). */
+ * adds left out, 186 us with this hand-over and the longer chunks of scan_steps).  The ring hex
+ * step writes out with emit_runs_ring instead. */
 template <class T, class W>
 __device__ __forceinline__ void emit_runs(bool out, int32_t key, const T v[3], W* dst,
                                           unsigned long long* ws, int lane)
@@ -391,15 +392,68 @@ __device__ __forceinline__ void emit_runs(bool out, int32_t key, const T v[3], W
     __syncwarp();
 }
 
+/* emit_runs for the 32-bit sums of the ring hex step with one substep, which every instruction
+ * counts in.  The sums go to shared memory with their cell in one 16-byte store.
+ *
+ * `emit` is what the warp found at the first sums it wrote that were not all zero.  In a planar
+ * flow no sum has three non-zero components, there are a third fewer adds, and direct ones, one
+ * instruction per component, are faster.  1e7 parcels on 128^3 cells from rest, conversion
+ * overlapped, us per step over 20, 100 and 500 steps: without a z component 223 / 224 / 224
+ * handed over, 221 / 219 / 217 by this rule, 216 / 216 / 215 added directly in a kernel that has
+ * no other way; with three components 226 / 227 handed over and by this rule, 249 direct.
+ * (The vote on every call costs the second flow 1 to 2 %; an instance of the whole tile for
+ * each of the two, 5 %.) */
+enum Emit { EMIT_UNKNOWN = 0, EMIT_HAND_OVER = 1, EMIT_DIRECT = 2 };
+
+__device__ __forceinline__ void emit_runs_ring(bool out, int32_t key, const int v[3],
+                                               unsigned long long* acc, unsigned long long* ws,
+                                               int lane, int& emit)
+{
+    if (emit == EMIT_UNKNOWN) {
+        const int nz = out ? (v[0] != 0) + (v[1] != 0) + (v[2] != 0) : 0;
+        const int most = __reduce_max_sync(FULL_MASK, nz);
+        if (most) emit = most == 3 ? EMIT_HAND_OVER : EMIT_DIRECT;
+    }
+    if (emit == EMIT_DIRECT) {
+        if (out) {
+            unsigned long long* const p = acc + 3 * (int64_t)key;
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (v[k]) red_add(p + k, (unsigned long long)(long long)v[k]);
+        }
+        return;
+    }
+    const unsigned outs = __ballot_sync(FULL_MASK, out);
+    if (out)
+        reinterpret_cast<int4*>(ws)[__popc(outs & ((1u << lane) - 1u))] =
+            make_int4(v[0], v[1], v[2], key);
+    __syncwarp();
+    const int items = 3 * __popc(outs);
+    const int* const s = reinterpret_cast<const int*>(ws);
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        const int i = lane + 32 * t;
+        if (i < items) {
+            const int r = (i * 43) >> 7;   /* i / 3, exact for i < 128 */
+            const int q = s[i + r];
+            unsigned long long* const p = acc + (3 * (int64_t)s[4 * r + 3] + (i - 3 * r));
+            if (q) red_add(p, (unsigned long long)(long long)q);
+        }
+    }
+    __syncwarp();
+}
+
 /* Final deposits of 32 consecutive parcels (one per lane, key < 0 = none): runs of equal
  * cells are summed with a segmented warp scan and the last lane of each run adds the sum.
  * The FP64 atomic mode sums its runs in FP64 the same way.
- * `ws`: this warp's dep_ws_words<DEP, V> words of shared memory. */
+ * `ws`: this warp's dep_ws_words<DEP, V> words of shared memory.  `emit`: emit_runs_ring's, for
+ * its caller. */
 template <int DEP, class V>
 __device__ __forceinline__ void deposit_warp(int32_t key, const V dep[3],
                                              unsigned long long* acc, double* src,
                                              const Quant& qp, int lane, AmaxT<V>& amax,
-                                             unsigned& ovf, unsigned long long* ws)
+                                             unsigned& ovf, unsigned long long* ws,
+                                             int* emit = nullptr)
 {
     if (DEP == DEP_PROBE) {
         if (key >= 0) {
@@ -492,7 +546,8 @@ __device__ __forceinline__ void deposit_warp(int32_t key, const V dep[3],
         if (narrow) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) q32[k] = seg_scan<STEPS>(q32[k], lane, segstart);
-            emit_runs(out, key, q32, acc, ws, lane);
+            if (emit) emit_runs_ring(out, key, q32, acc, ws, lane, *emit);
+            else emit_runs(out, key, q32, acc, ws, lane);
             return;
         }
 #pragma unroll

@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256, MinBlocks<V, ONE>::value) k_step(const St
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     constexpr bool DET = (DEP == DEP_DET1 || DEP == DEP_DET2);
 
-    __shared__ unsigned long long dep_ws[8][dep_ws_words<DEP, V>];
+    __shared__ __align__(16) unsigned long long dep_ws[8][dep_ws_words<DEP, V>];
     unsigned long long* const ws = dep_ws[threadIdx.x >> 5];
     grid_dep_launch();
     if (!ONE && sizeof(V) == 4 && a.phys.drag != 0) {   /* the table of x^0.687 serves the multi-substep loop */

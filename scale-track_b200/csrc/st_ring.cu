@@ -53,7 +53,7 @@ __device__ __forceinline__ void ring_slices(const StepArgs<P, V>& a, P* xs, P* y
                                             unsigned long long* acc, double* src,
                                             const Quant& qp, int lane, AmaxT<V>& amax,
                                             unsigned& ovf, unsigned& nlost,
-                                            unsigned long long* scr)
+                                            unsigned long long* scr, int& emit)
 {
     P X[RING_SPW], Y[RING_SPW], Z[RING_SPW];
     V Uv[RING_SPW], Vv[RING_SPW], Wv[RING_SPW], D[RING_SPW];
@@ -120,7 +120,8 @@ __device__ __forceinline__ void ring_slices(const StepArgs<P, V>& a, P* xs, P* y
                 ring_st<GLOBAL>(ws + j, vel[2]);
             }
         }
-        deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf, scr);
+        deposit_warp<DEP, V>(key, dep, acc, src, qp, lane, amax, ovf, scr,
+                             ONE && DEP == DEP_DET1 ? &emit : nullptr);
     }
 }
 
@@ -136,11 +137,12 @@ struct HexRing {
     unsigned& ovf;
     unsigned& nlost;
     unsigned long long* scr;
+    int emit = EMIT_UNKNOWN;   /* of this warp (emit_runs_ring) */
     template <bool GLOBAL>
     __device__ __forceinline__ void run(const RingArrays<P, V>& r, int j0, int64_t nvalid)
     {
         ring_slices<P, V, DEP, ONE, GLOBAL>(a, r.x, r.y, r.z, r.u, r.v, r.w, r.d, j0, nvalid, acc,
-                                            src, qp, lane, amax, ovf, nlost, scr);
+                                            src, qp, lane, amax, ovf, nlost, scr, emit);
     }
 };
 
@@ -157,7 +159,7 @@ __global__ void __launch_bounds__(HexShapeOf<V>::type::THREADS, 1)
     AmaxT<V> amax = (V)0;
     unsigned ovf = 0, nlost = 0;
     const int lane = threadIdx.x & 31;
-    __shared__ unsigned long long dep_ws[HexShape::CONS][dep_ws_words<DEP, V>];
+    __shared__ __align__(16) unsigned long long dep_ws[HexShape::CONS][dep_ws_words<DEP, V>];
     HexRing<P, V, DEP, ONE> step{a, DET ? a.one.acc : nullptr,
                                  DEP == DEP_ATOMIC ? a.one.src : nullptr, qp, lane, amax, ovf,
                                  nlost, dep_ws[min(threadIdx.x >> 5, HexShape::CONS - 1)]};

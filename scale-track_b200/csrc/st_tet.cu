@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(256, TetMinBlocks<V>::value) k_step_tet(const 
     unsigned ovf = 0, nlost = 0;
     const int nsub = ONE ? 1 : ph.nsub;
     const bool count_hops = a.hop_hist != nullptr && DEP != DEP_PROBE;
-    __shared__ unsigned long long dep_ws[8][dep_ws_words<DEP, V>];
+    __shared__ __align__(16) unsigned long long dep_ws[8][dep_ws_words<DEP, V>];
     unsigned long long* const ws = dep_ws[threadIdx.x >> 5];
     grid_dep_launch();
     grid_dep_wait();
@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(TetShape::THREADS, 1) k_step_tet_ring(const Te
     const bool count_hops = a.hop_hist != nullptr;
     if (threadIdx.x < 8) s_tet_hist[threadIdx.x] = 0;   /* ring_block synchronises */
     ring_emax_init();
-    __shared__ unsigned long long dep_ws[TetShape::CONS][dep_ws_words<DEP, V>];
+    __shared__ __align__(16) unsigned long long dep_ws[TetShape::CONS][dep_ws_words<DEP, V>];
     TetRing<V, DEP, ONE> step{a, DET ? a.one.acc : nullptr,
                               DEP == DEP_ATOMIC ? a.one.src : nullptr, qp, lane, count_hops,
                               amax, ovf, nlost,
