@@ -162,8 +162,6 @@ __device__ __forceinline__ int32_t tet_walk(const TetMeshK& m, int32_t t, const 
                      fabs(x[2]) <= (double)m.xmax;
     for (int it = 0; it <= hop_limit; ++it) {
         int fb = 0;
-        /* all four neighbours beside the planes: a hop then waits for one load, not two */
-        const int4 nbr = __ldg(reinterpret_cast<const int4*>(m.nbr) + t);
         const int r = pre ? tet_step32(m, t, x32, fb) : 0;
         if (r == 1) {
             status = TWALK_OK;
@@ -181,7 +179,10 @@ __device__ __forceinline__ int32_t tet_walk(const TetMeshK& m, int32_t t, const 
                 return t;
             }
         }
-        const int32_t nb = fb == 0 ? nbr.x : (fb == 1 ? nbr.y : (fb == 2 ? nbr.z : nbr.w));
+        /* one neighbour, once it is known which: all four beside the planes read 16 bytes more on
+         * every look, also of the walks that end there (5e6 unsorted parcels on 1.6e6 tets: 365
+         * us per launch beside the planes, 281 now; sorted 145 and 148) */
+        const int32_t nb = __ldg(m.nbr + 4 * (int64_t)t + fb);
         if (nb < 0) {
             status = TWALK_EXIT;
             return t;
@@ -412,9 +413,8 @@ __global__ void __launch_bounds__(256, TetMinBlocks<V>::value) k_step_tet(const 
  * bounds the step are the walk's chains of dependent gathers (owning tet's U and planes ->
  * neighbour -> its planes), which need many warps in flight and few requests per look: 2e7
  * parcels on 5.3e6 tets 720 us per launch; planes in 32-byte loads 705; nothing of a look in
- * local memory 627 (23 consumer warps 756, 27 679); neighbours loaded with the planes 609;
- * the first planes prefetched 599.  Without the walk it takes 341 us, without the deposits' adds
- * 75 us less.  Packing the unfinished walks of several slices into full warps was slower (768 at
+ * local memory 627 (23 consumer warps 756, 27 679); the first planes prefetched 620.  Without
+ * the walk it takes 341 us, without the deposits' adds 75 us less.  Packing the unfinished walks of several slices into full warps was slower (768 at
  * the same warps, 833 with two slices per warp), and so were prefetches for the next tile
  * (639). */
 using TetShape = RingShape<992, 31>;
