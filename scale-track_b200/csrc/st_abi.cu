@@ -367,6 +367,22 @@ int ensure_stage(st_handle* h, size_t bytes)
     return ST_OK;
 }
 
+/* ensure_stage for a caller that can do without: false, and the staging array as it was, when
+ * there is no memory for it. */
+bool try_stage(st_handle* h, size_t bytes)
+{
+    if (h->stage_bytes >= bytes) return true;
+    void* p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (h->dstage) cudaFree(h->dstage);
+    h->dstage = p;
+    h->stage_bytes = bytes;
+    return true;
+}
+
 /* Reads the control blocks; reports (and clears) lost parcels and range errors. */
 int check_device_errors(st_handle* h)
 {
@@ -742,29 +758,54 @@ int do_step_tet(st_handle* h, double dt, double fscale, int phase)
                        [&] { return do_sort_all<double, V>(h); });
 }
 
-/* Parcels pass between the caller's arrays and the cloud in chunks of this many, converted
- * and ordered on the device through the handle's staging array (59 MB). */
+/* Parcels pass between the caller's arrays and the cloud in chunks of at most this many,
+ * converted and ordered on the device. */
 constexpr int64_t PARCEL_CHUNK = (int64_t)1 << 20;
+
+int64_t even(int64_t n) { return n + (n & 1); }
+
+/* Where the chunks of m parcels are staged, in the caller's doubles, and how many at a time.  In
+ * the cloud's idle buffers (c.x[1 - cur] ..., free between steps), which takes no memory: an
+ * array of cap floats holds cap / 2 doubles, and cap is even.  Where that would cut a large
+ * transfer into more chunks, the handle's staging array instead (at most 59 MB), if there is
+ * memory for it: 1e6 FP32 parcels read back in one chunk 2.57 ms, in two 2.95 ms; a small cloud
+ * set without the allocation 0.57 -> 0.47 ms. */
+template <class V>
+int64_t parcel_stage(st_handle* h, const CloudBufs& c, int64_t m, ParcelStage& st)
+{
+    const int64_t want = std::min(m, PARCEL_CHUNK);
+    const int64_t idle = c.cap * (int64_t)sizeof(V) / (int64_t)sizeof(double);
+    const size_t bytes = (size_t)want * 7 * sizeof(double);
+    if (idle < want && bytes >= ((size_t)2 << 20) && try_stage(h, bytes)) {
+        double* const p = static_cast<double*>(h->dstage);
+        st = {p, p + want, p + 2 * want, p + 3 * want, p + 4 * want, p + 5 * want, p + 6 * want};
+        return want;
+    }
+    const int i = 1 - c.cur;
+    st = {(double*)c.x[i], (double*)c.y[i], (double*)c.z[i], (double*)c.u[i],
+          (double*)c.v[i], (double*)c.w[i], (double*)c.d[i]};
+    return std::min(want, idle);
+}
 
 /* The caller's [3][m], [3][m] and [m] arrays into the current buffers at first .. first+m-1. */
 template <class P, class V>
 int import_parcels(st_handle* h, CloudBufs& c, int64_t first, int64_t m, const double* xyz,
                    const double* uvw, const double* d)
 {
-    int rc;
-    if ((rc = ensure_stage(h, (size_t)std::min(m, PARCEL_CHUNK) * 7 * sizeof(double)))) return rc;
-    double* const st = static_cast<double*>(h->dstage);
+    ParcelStage ps;
+    const int64_t chunk = parcel_stage<V>(h, c, m, ps);
+    double* const st[7] = {ps.x, ps.y, ps.z, ps.u, ps.v, ps.w, ps.d};
     SortBufs<P, V> b = sort_bufs<P, V>(h, c);
-    for (int64_t o = 0; o < m; o += PARCEL_CHUNK) {
-        const int64_t k = std::min(PARCEL_CHUNK, m - o);
+    for (int64_t o = 0; o < m; o += chunk) {
+        const int64_t k = std::min(chunk, m - o);
         XferSeg seg[7];
         for (int a = 0; a < 7; ++a) {
             const double* src = (a < 3 ? xyz + a * m : (a < 6 ? uvw + (a - 3) * m : d)) + o;
-            seg[a] = {const_cast<double*>(src), st + a * k, k * sizeof(double)};
+            seg[a] = {const_cast<double*>(src), st[a], k * sizeof(double)};
         }
         CK(xfer_up(seg, 7, h->device, h->stream));
-        ProfScope ps(h, ST_KERNEL_OTHER);
-        CK(import_chunk<P, V>(b, c.cur, first + o, k, st, h->stream));
+        ProfScope scope(h, ST_KERNEL_OTHER);
+        CK(import_chunk<P, V>(b, c.cur, first + o, k, ps, h->stream));
         h->launches += 1;
     }
     return ST_OK;
@@ -782,6 +823,7 @@ int do_set_parcels(st_handle* h, int cloud, int64_t n, const double* xyz, const 
 {
     CloudBufs& c = h->clouds[cloud];
     if (n > c.cap) {
+        const int64_t cap = even(n);
         /* a failed allocation below leaves an empty cloud that the next call reallocates */
         c.cap = 0;
         c.n = 0;
@@ -791,7 +833,7 @@ int do_set_parcels(st_handle* h, int cloud, int64_t n, const double* xyz, const 
             for (int a = 0; a < 7; ++a) {
                 if (*arrs[a]) cudaFree(*arrs[a]);
                 *arrs[a] = nullptr;
-                CK(cudaMalloc(arrs[a], (size_t)n * (a < 3 ? sizeof(P) : sizeof(V))));
+                CK(cudaMalloc(arrs[a], (size_t)cap * (a < 3 ? sizeof(P) : sizeof(V))));
             }
             if (c.id[k]) cudaFree(c.id[k]);
             if (c.keys[k]) cudaFree(c.keys[k]);
@@ -800,12 +842,12 @@ int do_set_parcels(st_handle* h, int cloud, int64_t n, const double* xyz, const 
             c.id[k] = nullptr;
             c.cell[k] = nullptr;
             c.keys[k] = c.perm[k] = nullptr;
-            if (h->tet) CK(cudaMalloc(&c.cell[k], (size_t)n * sizeof(int32_t)));
-            CK(cudaMalloc(&c.id[k], (size_t)n * sizeof(int32_t)));
-            CK(cudaMalloc(&c.keys[k], (size_t)n * sizeof(uint32_t)));
-            CK(cudaMalloc(&c.perm[k], (size_t)n * sizeof(uint32_t)));
+            if (h->tet) CK(cudaMalloc(&c.cell[k], (size_t)cap * sizeof(int32_t)));
+            CK(cudaMalloc(&c.id[k], (size_t)cap * sizeof(int32_t)));
+            CK(cudaMalloc(&c.keys[k], (size_t)cap * sizeof(uint32_t)));
+            CK(cudaMalloc(&c.perm[k], (size_t)cap * sizeof(uint32_t)));
         }
-        c.cap = n;
+        c.cap = cap;
     }
     c.n = n;
     c.cur = 0;
@@ -879,7 +921,7 @@ int do_append_parcels(st_handle* h, int cloud, int64_t m, const double* xyz, con
     const int64_t n = c.n, nn = n + m;
     if (nn > c.cap) {
         int64_t cap = c.cap + c.cap / 2;
-        if (cap < nn) cap = nn;
+        cap = even(std::max(cap, nn));
         /* every new buffer is allocated before anything is replaced, so a failure leaves the
          * cloud as it was */
         void** arrs[2][8] = {{&c.x[0], &c.y[0], &c.z[0], &c.u[0], &c.v[0], &c.w[0], &c.d[0],
@@ -957,20 +999,20 @@ int do_get_parcels(st_handle* h, int cloud, double* xyz, double* uvw, double* d)
     CloudBufs& c = h->clouds[cloud];
     const int64_t n = c.n;
     if (n == 0) return ST_OK;
-    int rc;
-    if ((rc = ensure_stage(h, (size_t)std::min(n, PARCEL_CHUNK) * 7 * sizeof(double)))) return rc;
-    double* const st = static_cast<double*>(h->dstage);
+    ParcelStage ps;
+    const int64_t chunk = parcel_stage<V>(h, c, n, ps);
+    double* const st[7] = {ps.x, ps.y, ps.z, ps.u, ps.v, ps.w, ps.d};
     SortBufs<P, V> b = sort_bufs<P, V>(h, c);
     {
-        ProfScope ps(h, ST_KERNEL_OTHER);
+        ProfScope scope(h, ST_KERNEL_OTHER);
         CK(export_order<P, V>(b, c.cur, n, h->stream));
         h->launches += 1;
     }
-    for (int64_t o = 0; o < n; o += PARCEL_CHUNK) {
-        const int64_t k = std::min(PARCEL_CHUNK, n - o);
+    for (int64_t o = 0; o < n; o += chunk) {
+        const int64_t k = std::min(chunk, n - o);
         {
-            ProfScope ps(h, ST_KERNEL_OTHER);
-            CK(export_chunk<P, V>(b, c.cur, o, k, st, h->stream));
+            ProfScope scope(h, ST_KERNEL_OTHER);
+            CK(export_chunk<P, V>(b, c.cur, o, k, ps, h->stream));
             h->launches += 1;
         }
         XferSeg seg[7];
@@ -979,7 +1021,7 @@ int do_get_parcels(st_handle* h, int cloud, double* xyz, double* uvw, double* d)
             double* dst = a < 3 ? (xyz ? xyz + a * n + o : nullptr)
                                 : (a < 6 ? (uvw ? uvw + (a - 3) * n + o : nullptr)
                                          : (d ? d + o : nullptr));
-            if (dst) seg[ns++] = {dst, st + a * k, k * sizeof(double)};
+            if (dst) seg[ns++] = {dst, st[a], k * sizeof(double)};
         }
         CK(xfer_down(seg, ns, h->device, h->stream));
     }

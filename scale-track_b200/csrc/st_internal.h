@@ -360,17 +360,21 @@ size_t count_sort_scan_bytes(int key_bits);
 template <class P, class V>
 cudaError_t sort_cloud(SortBufs<P, V>& b, int cur, int64_t n, const MeshK<P>& mesh, int key_bits,
                        int key_shift, bool morton, cudaStream_t s, int* launches);
-/* Parcels to and from the caller's layout (FP64, order of st_set_parcels), a chunk of m
- * parcels from index `base` at a time as [7][m] (x, y, z, u, v, w, d).  export_order first:
- * it leaves the inverse of the ids in b.perm[0] for the export_chunk calls. */
+/* Device staging of parcels as the caller holds them: FP64, an array per component. */
+struct ParcelStage {
+    double *x, *y, *z, *u, *v, *w, *d;
+};
+/* Parcels to and from the caller's layout (order of st_set_parcels), a chunk of m parcels from
+ * index `base` at a time.  export_order first: it leaves the inverse of the ids in b.perm[0] for
+ * the export_chunk calls. */
 template <class P, class V>
 cudaError_t export_order(SortBufs<P, V>& b, int cur, int64_t n, cudaStream_t s);
 template <class P, class V>
-cudaError_t export_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m, double* out,
-                         cudaStream_t s);
+cudaError_t export_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m,
+                         const ParcelStage& st, cudaStream_t s);
 template <class P, class V>
-cudaError_t import_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m, const double* in,
-                         cudaStream_t s);
+cudaError_t import_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m,
+                         const ParcelStage& st, cudaStream_t s);
 cudaError_t cells_unpermute(const int32_t* id, const int32_t* cell, int64_t n, int32_t* out,
                             cudaStream_t s);
 /* State ([6][m] FP64) and owning cells of the parcels ids[0..m) (st_set_parcels indices,

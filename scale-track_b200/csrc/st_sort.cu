@@ -148,45 +148,45 @@ __global__ void __launch_bounds__(256) k_gather(const uint32_t* __restrict__ per
     }
 }
 
-/* Parcels base .. base + m - 1 of the st_set_parcels order as the caller holds them: out =
- * [7][m] FP64 (x, y, z, u, v, w, d).  inv: k_inverse_ids. */
+/* Parcels base .. base + m - 1 of the st_set_parcels order as the caller holds them, one FP64
+ * array per component.  inv: k_inverse_ids. */
 template <class P, class V>
 __global__ void k_export(const uint32_t* __restrict__ inv, int64_t base, int64_t m,
                          const P* __restrict__ x, const P* __restrict__ y,
                          const P* __restrict__ z, const V* __restrict__ u,
                          const V* __restrict__ v, const V* __restrict__ w,
-                         const V* __restrict__ d, double* __restrict__ out)
+                         const V* __restrict__ d, ParcelStage out)
 {
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m;
          j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t p = inv[base + j];
-        out[j] = (double)x[p];
-        out[m + j] = (double)y[p];
-        out[2 * m + j] = (double)z[p];
-        out[3 * m + j] = (double)u[p];
-        out[4 * m + j] = (double)v[p];
-        out[5 * m + j] = (double)w[p];
-        out[6 * m + j] = (double)d[p];
+        out.x[j] = (double)x[p];
+        out.y[j] = (double)y[p];
+        out.z[j] = (double)z[p];
+        out.u[j] = (double)u[p];
+        out.v[j] = (double)v[p];
+        out.w[j] = (double)w[p];
+        out.d[j] = (double)d[p];
     }
 }
 
-/* The reverse: in = [7][m] FP64 into the arrays at base .. base + m - 1, with their ids. */
+/* The reverse: m staged parcels into the arrays at base .. base + m - 1, with their ids. */
 template <class P, class V>
-__global__ void k_import(const double* __restrict__ in, int64_t base, int64_t m,
-                         P* __restrict__ x, P* __restrict__ y, P* __restrict__ z,
-                         V* __restrict__ u, V* __restrict__ v, V* __restrict__ w,
-                         V* __restrict__ d, int32_t* __restrict__ id)
+__global__ void k_import(ParcelStage in, int64_t base, int64_t m, P* __restrict__ x,
+                         P* __restrict__ y, P* __restrict__ z, V* __restrict__ u,
+                         V* __restrict__ v, V* __restrict__ w, V* __restrict__ d,
+                         int32_t* __restrict__ id)
 {
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < m;
          j += (int64_t)gridDim.x * blockDim.x) {
         const int64_t p = base + j;
-        x[p] = (P)in[j];
-        y[p] = (P)in[m + j];
-        z[p] = (P)in[2 * m + j];
-        u[p] = (V)in[3 * m + j];
-        v[p] = (V)in[4 * m + j];
-        w[p] = (V)in[5 * m + j];
-        d[p] = (V)in[6 * m + j];
+        x[p] = (P)in.x[j];
+        y[p] = (P)in.y[j];
+        z[p] = (P)in.z[j];
+        u[p] = (V)in.u[j];
+        v[p] = (V)in.v[j];
+        w[p] = (V)in.w[j];
+        d[p] = (V)in.d[j];
         id[p] = (int32_t)p;
     }
 }
@@ -492,20 +492,22 @@ cudaError_t export_order(SortBufs<P, V>& b, int cur, int64_t n, cudaStream_t s)
 }
 
 template <class P, class V>
-cudaError_t export_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m, double* out,
-                         cudaStream_t s)
+cudaError_t export_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m,
+                         const ParcelStage& st, cudaStream_t s)
 {
     k_export<P, V><<<grid_for(m), 256, 0, s>>>(b.perm[0], base, m, b.x[cur], b.y[cur], b.z[cur],
-                                               b.u[cur], b.v[cur], b.w[cur], b.d[cur], out);
+                                               b.u[cur], b.v[cur], b.w[cur], b.d[cur],
+                                               st);
     return cudaGetLastError();
 }
 
 template <class P, class V>
-cudaError_t import_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m, const double* in,
-                         cudaStream_t s)
+cudaError_t import_chunk(SortBufs<P, V>& b, int cur, int64_t base, int64_t m,
+                         const ParcelStage& st, cudaStream_t s)
 {
-    k_import<P, V><<<grid_for(m), 256, 0, s>>>(in, base, m, b.x[cur], b.y[cur], b.z[cur],
-                                               b.u[cur], b.v[cur], b.w[cur], b.d[cur], b.id[cur]);
+    k_import<P, V><<<grid_for(m), 256, 0, s>>>(st, base, m, b.x[cur], b.y[cur],
+                                               b.z[cur], b.u[cur], b.v[cur], b.w[cur], b.d[cur],
+                                               b.id[cur]);
     return cudaGetLastError();
 }
 
@@ -545,10 +547,10 @@ cudaError_t cells_unpermute(const int32_t* id, const int32_t* cell, int64_t n, i
     template cudaError_t sort_cloud<P, V>(SortBufs<P, V>&, int, int64_t, const MeshK<P>&, int, \
                                           int, bool, cudaStream_t, int*);                     \
     template cudaError_t export_order<P, V>(SortBufs<P, V>&, int, int64_t, cudaStream_t);      \
-    template cudaError_t export_chunk<P, V>(SortBufs<P, V>&, int, int64_t, int64_t, double*,    \
-                                            cudaStream_t);                                     \
+    template cudaError_t export_chunk<P, V>(SortBufs<P, V>&, int, int64_t, int64_t,             \
+                                            const ParcelStage&, cudaStream_t);                 \
     template cudaError_t import_chunk<P, V>(SortBufs<P, V>&, int, int64_t, int64_t,             \
-                                            const double*, cudaStream_t);                      \
+                                            const ParcelStage&, cudaStream_t);                 \
     template cudaError_t sample_cloud<P, V>(SortBufs<P, V>&, int, int64_t, const MeshK<P>&,    \
                                             const int32_t*, int64_t, double*, int32_t*,        \
                                             cudaStream_t);
