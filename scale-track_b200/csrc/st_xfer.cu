@@ -15,7 +15,8 @@
  * The staging buffers belong to the process: XFER_THREADS pinned pieces (24 MB), made by the
  * first copy of XFER_MIN bytes or more and freed with the last handle.  One copy uses them at a
  * time; a copy that finds them taken (another host thread's), or cannot have them, and copies
- * to pinned memory or below XFER_MIN, go through plain cudaMemcpyAsync.
+ * to pinned memory or below XFER_MIN, go through plain cudaMemcpyAsync, and so do those of a
+ * handle in a context other than the device's primary one.
  */
 #include <atomic>
 #include <cstring>
@@ -60,13 +61,69 @@ cudaError_t plain(const XferSeg* seg, int n, bool down, cudaStream_t s)
     return cudaStreamSynchronize(s);
 }
 
-/* Takes pieces from the shared counter until none is left or a copy failed. */
+/* Whether the device's primary context is current on this thread.  The staging buffers and the
+ * helper threads (cudaSetDevice) are the primary context's; a caller that made its handle in a
+ * context of its own (driver API) has its copies on its own thread. */
+bool primary_current(int device)
+{
+    using DeviceGet = int (*)(int*, int);
+    using GetCurrent = int (*)(void**);
+    using GetState = int (*)(int, unsigned*, int*);
+    using Retain = int (*)(void**, int);
+    using Release = int (*)(int);
+    struct Api {
+        DeviceGet device = nullptr;
+        GetCurrent current = nullptr;
+        GetState state = nullptr;
+        Retain retain = nullptr;
+        Release release = nullptr;
+        static void* find(const char* name)
+        {
+            void* f = nullptr;
+            cudaDriverEntryPointQueryResult r;
+            if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &r) != cudaSuccess ||
+                r != cudaDriverEntryPointSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            return f;
+        }
+        Api()
+        {
+            device = reinterpret_cast<DeviceGet>(find("cuDeviceGet"));
+            current = reinterpret_cast<GetCurrent>(find("cuCtxGetCurrent"));
+            state = reinterpret_cast<GetState>(find("cuDevicePrimaryCtxGetState"));
+            retain = reinterpret_cast<Retain>(find("cuDevicePrimaryCtxRetain"));
+            release = reinterpret_cast<Release>(find("cuDevicePrimaryCtxRelease"));
+        }
+    };
+    static const Api api;
+    if (!api.device || !api.current || !api.state || !api.retain || !api.release) return false;
+    void *now = nullptr, *primary = nullptr;
+    unsigned flags = 0;
+    int dev = 0, active = 0;
+    /* (retaining an inactive primary context would make it) */
+    if (api.device(&dev, device) || api.current(&now) || api.state(dev, &flags, &active) ||
+        !active || api.retain(&primary, dev))
+        return false;
+    api.release(dev);
+    return now == primary;
+}
+
+/* Takes pieces from the shared counter until none is left or a copy failed.  `helper`: on a
+ * thread of its own, which first needs the device; where it does not get it, or cannot work on
+ * the stream, it leaves the pieces to the others. */
 void worker(const std::vector<Piece>& pieces, std::atomic<size_t>& next, std::atomic<int>& err,
-            unsigned char* pin, bool down, int device, cudaStream_t s)
+            unsigned char* pin, bool down, int device, cudaStream_t s, bool helper)
 {
     cudaEvent_t ev = nullptr;
-    cudaError_t e = cudaSetDevice(device);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    cudaError_t e = cudaSuccess;
+    if (helper && cudaSetDevice(device) != cudaSuccess) return;
+    e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (helper && (e != cudaSuccess || cudaEventRecord(ev, s) != cudaSuccess)) {
+        if (ev) cudaEventDestroy(ev);
+        return;
+    }
     while (e == cudaSuccess && err.load() == (int)cudaSuccess) {
         const size_t k = next.fetch_add(1);
         if (k >= pieces.size()) break;
@@ -105,7 +162,8 @@ cudaError_t xfer(const XferSeg* seg, int n, bool down, int device, cudaStream_t 
         for (int k = 0; k < n; ++k) pageable = pageable || !pinned(seg[k].host);
     std::unique_lock<std::mutex> lk(g_pin_mu, std::defer_lock);
     /* (the per-thread stream is another one on every thread) */
-    if (!pageable || s == cudaStreamPerThread || !lk.try_lock()) return plain(seg, n, down, s);
+    if (!pageable || s == cudaStreamPerThread || !primary_current(device) || !lk.try_lock())
+        return plain(seg, n, down, s);
     if (!g_pin && cudaHostAlloc((void**)&g_pin, XFER_THREADS * XFER_PIECE, cudaHostAllocPortable) !=
                       cudaSuccess) {
         cudaGetLastError();
@@ -138,12 +196,12 @@ cudaError_t xfer(const XferSeg* seg, int n, bool down, int device, cudaStream_t 
     for (int t = 1; t < nt; ++t) {
         try {
             ts.emplace_back(worker, std::cref(pieces), std::ref(next), std::ref(err),
-                            g_pin + t * XFER_PIECE, down, device, s);
+                            g_pin + t * XFER_PIECE, down, device, s, true);
         } catch (...) {
             break;                             /* no more threads: fewer take the pieces */
         }
     }
-    worker(pieces, next, err, g_pin, down, device, s);
+    worker(pieces, next, err, g_pin, down, device, s, false);
     for (std::thread& t : ts) t.join();
     return (cudaError_t)err.load();
 }

@@ -1,0 +1,111 @@
+"""CPU test of the staged host copies (st_xfer.cu) on a stand-in for the CUDA runtime: bytes, which
+contexts the copies touch."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+DRIVER = r"""
+#include <cassert>
+#include <cstdio>
+#include <thread>
+#include <vector>
+#include "st_xfer.h"
+
+namespace fake {
+std::atomic<int> set_device{0}, host_allocs{0}, copies{0}, syncs{0}, fail_copy{0};
+std::atomic<long> host_bytes{0};
+thread_local void* context = nullptr;
+thread_local int mode = cudaStreamCaptureModeGlobal;
+int primary_word, other_word;
+void *primary = &primary_word, *stream_context = &primary_word;
+bool refuse_alloc = false;
+int global_capture = 0;
+std::mutex mu;
+std::set<void*> pinned;
+}  // namespace fake
+using namespace st;
+
+static const size_t MB = (size_t)1 << 20;
+
+/* Both directions of `bytes` bytes in three segments of odd sizes; whether all arrived. */
+static bool both(size_t bytes, cudaError_t* err = nullptr)
+{
+    std::vector<unsigned char> a(bytes), dev(bytes, 0), b(bytes, 0);
+    for (size_t i = 0; i < bytes; ++i) a[i] = (unsigned char)(i * 2654435761u >> 13);
+    const size_t c1 = bytes / 3 | 1, c2 = bytes / 2 | 1;
+    auto seg = [&](unsigned char* h, XferSeg* s) {
+        s[0] = {h, dev.data(), c1};
+        s[1] = {h + c1, dev.data() + c1, c2 - c1};
+        s[2] = {h + c2, dev.data() + c2, bytes - c2};
+    };
+    XferSeg s[3];
+    int stream = 0;
+    seg(a.data(), s);
+    cudaError_t e = xfer_up(s, 3, 0, &stream);
+    seg(b.data(), s);
+    if (e == cudaSuccess) e = xfer_down(s, 3, 0, &stream);
+    if (err) *err = e;
+    return e == cudaSuccess && a == b && a == dev;
+}
+
+int main(int argc, char** argv)
+{
+    const std::string what = argv[1];
+    fake::context = fake::primary;
+    xfer_retain();
+    if (what == "bytes") {
+        for (size_t n : {(size_t)9, 2 * MB - 1, 2 * MB, 3 * MB + 5, 16 * MB - 7, 40 * MB + 3, 100 * MB + 1})
+            assert(both(n));
+        std::thread t([] {
+            fake::context = fake::primary;
+            for (int k = 0; k < 20; ++k) assert(both(7 * MB + k));
+        });
+        for (int k = 0; k < 20; ++k) assert(both(9 * MB + k));
+        t.join();
+    } else if (what == "own_context") {
+        /* a handle in a context of the caller's: its copies arrive and its context stays */
+        fake::context = fake::stream_context = &fake::other_word;
+        assert(both(100 * MB));
+        assert(fake::context == &fake::other_word && fake::set_device == 0);
+        /* and one in the primary context afterwards */
+        fake::context = fake::stream_context = fake::primary;
+        assert(both(100 * MB));
+    } else if (what == "no_primary") {
+        fake::primary = nullptr;
+        fake::context = fake::stream_context = &fake::other_word;
+        assert(both(30 * MB) && fake::context == &fake::other_word);
+    } else if (what == "no_pinned") {
+        fake::refuse_alloc = true;
+        assert(both(100 * MB));
+    } else {
+        return 2;
+    }
+    xfer_release();
+    assert(fake::pinned.empty());
+    puts("ok");
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def driver(tmp_path_factory):
+    d = tmp_path_factory.mktemp("xfer")
+    src = d / "driver.cpp"
+    src.write_text("#include <string>\n" + DRIVER)
+    exe = d / "driver"
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-pthread", "-I",
+                           os.path.join(ROOT, "tests", "fake_cuda"), "-I",
+                           os.path.join(ROOT, "scale-track_b200", "csrc"), str(src), "-x", "c++",
+                           os.path.join(ROOT, "scale-track_b200", "csrc", "st_xfer.cu"), "-o",
+                           str(exe)])
+    return str(exe)
+
+
+@pytest.mark.parametrize("what", ["bytes", "own_context", "no_primary", "no_pinned"])
+def test_staged_copies(driver, what):
+    r = subprocess.run([driver, what], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout == "ok\n", r.stderr
