@@ -118,7 +118,13 @@ void worker(const std::vector<Piece>& pieces, std::atomic<size_t>& next, std::at
 {
     cudaEvent_t ev = nullptr;
     cudaError_t e = cudaSuccess;
-    if (helper && cudaSetDevice(device) != cudaSuccess) return;
+    if (helper) {
+        /* what its copies may do is the caller's affair, not a capture's on another thread */
+        cudaStreamCaptureMode relaxed = cudaStreamCaptureModeRelaxed;
+        if (cudaThreadExchangeStreamCaptureMode(&relaxed) != cudaSuccess ||
+            cudaSetDevice(device) != cudaSuccess)
+            return;
+    }
     e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     if (helper && (e != cudaSuccess || cudaEventRecord(ev, s) != cudaSuccess)) {
         if (ev) cudaEventDestroy(ev);

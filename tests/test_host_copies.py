@@ -1,5 +1,5 @@
 """CPU test of the staged host copies (st_xfer.cu) on a stand-in for the CUDA runtime: bytes, which
-contexts the copies touch."""
+contexts the copies touch, captures on other threads."""
 import os
 import subprocess
 
@@ -77,6 +77,13 @@ int main(int argc, char** argv)
         fake::primary = nullptr;
         fake::context = fake::stream_context = &fake::other_word;
         assert(both(30 * MB) && fake::context == &fake::other_word);
+    } else if (what == "capture") {
+        /* another thread captures in global mode, and the caller's may copy all the same */
+        assert(both(100 * MB));
+        fake::global_capture = 1;
+        fake::mode = cudaStreamCaptureModeRelaxed;
+        for (int k = 0; k < 5; ++k) assert(both(100 * MB));
+        assert(fake::mode == cudaStreamCaptureModeRelaxed);
     } else if (what == "no_pinned") {
         fake::refuse_alloc = true;
         assert(both(100 * MB));
@@ -105,7 +112,7 @@ def driver(tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("what", ["bytes", "own_context", "no_primary", "no_pinned"])
+@pytest.mark.parametrize("what", ["bytes", "own_context", "no_primary", "capture", "no_pinned"])
 def test_staged_copies(driver, what):
     r = subprocess.run([driver, what], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout == "ok\n", r.stderr
