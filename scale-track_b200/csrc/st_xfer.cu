@@ -209,6 +209,7 @@ cudaError_t xfer(const XferSeg* seg, int n, bool down, int device, cudaStream_t 
     }
     worker(pieces, next, err, g_pin, down, device, s, false);
     for (std::thread& t : ts) t.join();
+    if (err.load() != (int)cudaSuccess) cudaStreamSynchronize(s);   /* no copy left in flight */
     return (cudaError_t)err.load();
 }
 

@@ -1,5 +1,5 @@
 """CPU test of the staged host copies (st_xfer.cu) on a stand-in for the CUDA runtime: bytes, which
-contexts the copies touch, captures on other threads."""
+threads and contexts the copies touch, failing calls."""
 import os
 import subprocess
 
@@ -87,6 +87,17 @@ int main(int argc, char** argv)
     } else if (what == "no_pinned") {
         fake::refuse_alloc = true;
         assert(both(100 * MB));
+    } else if (what == "failing_copy") {
+        assert(both(100 * MB));
+        for (int k = 1; k < 30; k += 4) {
+            fake::copies = 0;
+            fake::fail_copy = k;
+            cudaError_t e;
+            const int synced = fake::syncs;
+            assert(!both(30 * MB, &e) && e == cudaErrorUnknown && fake::syncs > synced);
+            fake::fail_copy = 0;
+            assert(both(30 * MB));
+        }
     } else {
         return 2;
     }
@@ -112,7 +123,8 @@ def driver(tmp_path_factory):
     return str(exe)
 
 
-@pytest.mark.parametrize("what", ["bytes", "own_context", "no_primary", "capture", "no_pinned"])
+@pytest.mark.parametrize("what", ["bytes", "own_context", "no_primary", "capture", "no_pinned",
+                                  "failing_copy"])
 def test_staged_copies(driver, what):
     r = subprocess.run([driver, what], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout == "ok\n", r.stderr
