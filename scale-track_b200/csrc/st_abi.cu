@@ -803,7 +803,7 @@ int import_parcels(st_handle* h, CloudBufs& c, int64_t first, int64_t m, const d
             const double* src = (a < 3 ? xyz + a * m : (a < 6 ? uvw + (a - 3) * m : d)) + o;
             seg[a] = {const_cast<double*>(src), st[a], k * sizeof(double)};
         }
-        CK(xfer_up(seg, 7, h->device, h->stream));
+        CK(xfer_up(seg, 7, h->device, h->stream, (size_t)(m - o - k) * 7 * sizeof(double)));
         ProfScope scope(h, ST_KERNEL_OTHER);
         CK(import_chunk<P, V>(b, c.cur, first + o, k, ps, h->stream));
         h->launches += 1;
@@ -1023,7 +1023,7 @@ int do_get_parcels(st_handle* h, int cloud, double* xyz, double* uvw, double* d)
                                          : (d ? d + o : nullptr));
             if (dst) seg[ns++] = {dst, st[a], k * sizeof(double)};
         }
-        CK(xfer_down(seg, ns, h->device, h->stream));
+        CK(xfer_down(seg, ns, h->device, h->stream, (size_t)(n - o - k) * ns * sizeof(double)));
     }
     return ST_OK;
 }

@@ -12,12 +12,19 @@
  * 162 -> 30 ms, an adjoint pass with 124 MB in and out 18.6 -> 10.7 ms, a 64^3 coupled step
  * with double fields 0.78 -> 0.75 ms.
  *
- * The staging buffers belong to the process: XFER_THREADS pinned pieces (24 MB), made by the
- * first copy of XFER_MIN bytes or more and freed with the last handle.  One copy uses them at a
- * time; a copy that finds them taken (another host thread's), or cannot have them, and copies
- * to pinned memory or below XFER_MIN, go through plain cudaMemcpyAsync, and so do those of a
- * handle in a context other than the device's primary one.
+ * The staging buffer belongs to the process: a pinned piece for each thread that a copy has work
+ * for, at most XFER_THREADS (24 MB), made when a copy first needs it and freed with the last
+ * handle.  Pinning is dear (16 ms for 24 MB, 2.5 ms to free), so copies go through plain
+ * cudaMemcpyAsync until XFER_RENT bytes have been copied, by when the staged copies would have
+ * saved about as much (0.04 ms per MB up, 0.16 down into pages that are used again).  So a
+ * program of small copies, or of one handle after another, does not pay for it each time (a fresh
+ * handle's 1e5 FP64 parcels set 23 ms when the first copy of 2 MB made the buffer, 3.0 ms now, the
+ * handle destroyed 5.9 and 2.8 ms; 1e6 FP32 parcels 28 and 12 ms, 11.5 and 7.7 ms).  One copy
+ * uses the buffer at a time; a copy that finds it taken (another host thread's), or cannot have
+ * it, and copies to pinned memory or below XFER_MIN, go through plain cudaMemcpyAsync, and so do
+ * those of a handle in a context other than the device's primary one.
  */
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <cstdint>
@@ -31,17 +38,21 @@
 namespace st {
 namespace {
 
-/* 2 MB pieces, 1 MB below 16 MB in all (three 2 MB pieces would leave threads without one):
- * the read-back above 3.03 -> 2.85 ms; pieces of 256 KB 3.5 ms.  Twelve threads against eight:
- * 50 MB into fresh pages 3.43 -> 3.02 ms, sixteen 3.74 ms. */
+/* 2 MB pieces (1 MB: 1e6 parcels read back in 2.90 against 2.37 ms; 256 KB 3.5 ms), 1 MB below
+ * 16 MB in all (three 2 MB pieces would leave threads without one: a 64^3 coupled step 0.81
+ * against 0.70 ms).  Twelve threads against eight: 50 MB into fresh pages 3.43 -> 3.02 ms,
+ * sixteen 3.74 ms. */
 constexpr size_t XFER_PIECE = (size_t)2 << 20;
 constexpr size_t XFER_MIN = (size_t)2 << 20;
+constexpr size_t XFER_RENT = (size_t)128 << 20;
 constexpr int XFER_THREADS = 12;
 
 std::mutex g_users_mu;
 int g_users = 0;             /* live handles */
-std::mutex g_pin_mu;         /* held by the copy that uses the buffers */
-unsigned char* g_pin = nullptr;   /* [XFER_THREADS][XFER_PIECE], pinned */
+std::mutex g_pin_mu;         /* held by the copy that uses the buffer */
+unsigned char* g_pin = nullptr;   /* [g_pieces][XFER_PIECE], pinned */
+int g_pieces = 0;
+size_t g_copied = 0;         /* bytes copied since the buffer was last given back */
 
 struct Piece {
     unsigned char* host;
@@ -159,7 +170,33 @@ bool pinned(const void* p)
     return at.type != cudaMemoryTypeUnregistered;
 }
 
-cudaError_t xfer(const XferSeg* seg, int n, bool down, int device, cudaStream_t s)
+void give_back()
+{
+    if (g_pin) cudaFreeHost(g_pin);
+    g_pin = nullptr;
+    g_pieces = 0;
+}
+
+/* Pinned pieces for nt threads, or for as many as there are when no more can be had. */
+int have_pieces(int nt)
+{
+    if (g_pin && !pinned(g_pin)) {        /* gone with a reset device */
+        g_pin = nullptr;
+        g_pieces = 0;
+    }
+    if (g_pieces >= nt) return nt;
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, nt * XFER_PIECE, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return g_pieces;
+    }
+    give_back();
+    g_pin = static_cast<unsigned char*>(p);
+    return g_pieces = nt;
+}
+
+cudaError_t xfer(const XferSeg* seg, int n, bool down, int device, cudaStream_t s,
+                 size_t ahead)
 {
     size_t total = 0;
     bool pageable = false;
@@ -170,16 +207,13 @@ cudaError_t xfer(const XferSeg* seg, int n, bool down, int device, cudaStream_t 
     /* (the per-thread stream is another one on every thread) */
     if (!pageable || s == cudaStreamPerThread || !primary_current(device) || !lk.try_lock())
         return plain(seg, n, down, s);
-    if (!g_pin && cudaHostAlloc((void**)&g_pin, XFER_THREADS * XFER_PIECE, cudaHostAllocPortable) !=
-                      cudaSuccess) {
-        cudaGetLastError();
-        g_pin = nullptr;
-        return plain(seg, n, down, s);
-    }
+    g_copied += total;
+    if (g_copied + ahead < XFER_RENT) return plain(seg, n, down, s);
     const int cores = (int)std::thread::hardware_concurrency();
-    int nt = (int)(total / XFER_MIN) + 1;      /* a thread costs about 20 us: 2 MB each at least */
+    int nt = (int)(total / XFER_MIN) + 1;      /* a thread costs about 20 us: 1 MB each at least */
     if (nt > XFER_THREADS) nt = XFER_THREADS;
     if (cores > 0 && nt > cores) nt = cores;
+    if ((nt = have_pieces(nt)) == 0) return plain(seg, n, down, s);
     const size_t piece = total >= 8 * XFER_PIECE ? XFER_PIECE : XFER_PIECE / 2;
     std::vector<Piece> pieces;
     std::vector<std::thread> ts;
@@ -193,7 +227,7 @@ cudaError_t xfer(const XferSeg* seg, int n, bool down, int device, cudaStream_t 
         unsigned char* hp = static_cast<unsigned char*>(seg[k].host);
         unsigned char* dp = static_cast<unsigned char*>(seg[k].dev);
         for (size_t o = 0; o < seg[k].bytes; o += piece) {
-            const size_t b = seg[k].bytes - o < piece ? seg[k].bytes - o : piece;
+            const size_t b = std::min(seg[k].bytes - o, piece);
             pieces.push_back({hp + o, dp + o, b});
         }
     }
@@ -215,14 +249,14 @@ cudaError_t xfer(const XferSeg* seg, int n, bool down, int device, cudaStream_t 
 
 }  // namespace
 
-cudaError_t xfer_down(const XferSeg* seg, int n, int device, cudaStream_t s)
+cudaError_t xfer_down(const XferSeg* seg, int n, int device, cudaStream_t s, size_t ahead)
 {
-    return xfer(seg, n, true, device, s);
+    return xfer(seg, n, true, device, s, ahead);
 }
 
-cudaError_t xfer_up(const XferSeg* seg, int n, int device, cudaStream_t s)
+cudaError_t xfer_up(const XferSeg* seg, int n, int device, cudaStream_t s, size_t ahead)
 {
-    return xfer(seg, n, false, device, s);
+    return xfer(seg, n, false, device, s, ahead);
 }
 
 void xfer_retain()
@@ -236,8 +270,8 @@ void xfer_release()
     std::lock_guard<std::mutex> lk(g_users_mu);
     if (--g_users > 0) return;
     std::lock_guard<std::mutex> pin(g_pin_mu);
-    if (g_pin) cudaFreeHost(g_pin);
-    g_pin = nullptr;
+    give_back();
+    g_copied = 0;
 }
 
 }  // namespace st

@@ -17,11 +17,12 @@ struct XferSeg {
 };
 
 /* Copies the segments in the order of stream `s` and returns when they have arrived (down:
- * device to host, up: host to device).  Call with `device` current. */
-cudaError_t xfer_down(const XferSeg* seg, int n, int device, cudaStream_t s);
-cudaError_t xfer_up(const XferSeg* seg, int n, int device, cudaStream_t s);
+ * device to host, up: host to device).  Call with `device` current.  ahead: bytes that the caller
+ * goes on to copy in the same call. */
+cudaError_t xfer_down(const XferSeg* seg, int n, int device, cudaStream_t s, size_t ahead = 0);
+cudaError_t xfer_up(const XferSeg* seg, int n, int device, cudaStream_t s, size_t ahead = 0);
 
-/* The pinned staging buffers are shared by the process: made by the first large copy, given
+/* The pinned staging buffer is shared by the process: made once enough has been copied, given
  * back when the last handle is destroyed. */
 void xfer_retain();
 void xfer_release();

@@ -1,5 +1,5 @@
 """CPU test of the staged host copies (st_xfer.cu) on a stand-in for the CUDA runtime: bytes, which
-threads and contexts the copies touch, failing calls."""
+contexts the copies touch, captures on other threads, what is pinned, failing calls."""
 import os
 import subprocess
 
@@ -56,8 +56,10 @@ int main(int argc, char** argv)
     const std::string what = argv[1];
     fake::context = fake::primary;
     xfer_retain();
+    if (what != "on_demand" && what != "no_primary" && what != "own_context")
+        assert(both(140 * MB));             /* copies are staged from now on */
     if (what == "bytes") {
-        for (size_t n : {(size_t)9, 2 * MB - 1, 2 * MB, 3 * MB + 5, 16 * MB - 7, 40 * MB + 3, 100 * MB + 1})
+        for (size_t n : {(size_t)9, 140 * MB, 2 * MB - 1, 2 * MB, 3 * MB + 5, 16 * MB - 7, 40 * MB + 3, 100 * MB + 1})
             assert(both(n));
         std::thread t([] {
             fake::context = fake::primary;
@@ -68,15 +70,16 @@ int main(int argc, char** argv)
     } else if (what == "own_context") {
         /* a handle in a context of the caller's: its copies arrive and its context stays */
         fake::context = fake::stream_context = &fake::other_word;
-        assert(both(100 * MB));
+        assert(both(300 * MB));
         assert(fake::context == &fake::other_word && fake::set_device == 0);
         /* and one in the primary context afterwards */
         fake::context = fake::stream_context = fake::primary;
-        assert(both(100 * MB));
+        assert(both(300 * MB));
+        assert(fake::set_device > 0);
     } else if (what == "no_primary") {
         fake::primary = nullptr;
         fake::context = fake::stream_context = &fake::other_word;
-        assert(both(30 * MB) && fake::context == &fake::other_word);
+        assert(both(300 * MB) && fake::context == &fake::other_word);
     } else if (what == "capture") {
         /* another thread captures in global mode, and the caller's may copy all the same */
         assert(both(100 * MB));
@@ -85,7 +88,42 @@ int main(int argc, char** argv)
         for (int k = 0; k < 5; ++k) assert(both(100 * MB));
         assert(fake::mode == cudaStreamCaptureModeRelaxed);
     } else if (what == "no_pinned") {
+        xfer_release();
+        xfer_retain();
         fake::refuse_alloc = true;
+        assert(both(300 * MB));
+    } else if (what == "on_demand") {
+        /* nothing is pinned for small copies, or before 128 MB have been copied; then only what
+         * the copy's threads use, at most 24 MB; and all of it goes with the last handle */
+        for (int k = 0; k < 200; ++k) assert(both(2 * MB - 1));
+        assert(fake::host_allocs == 0);
+        for (int k = 0; k < 12; ++k) assert(both(5 * MB));
+        assert(fake::host_allocs == 0);
+        for (int k = 0; k < 5; ++k) assert(both(5 * MB));
+        assert(fake::host_bytes > 0 && fake::host_bytes <= (long)(6 * MB));
+        xfer_retain();
+        for (int k = 0; k < 3; ++k) assert(both(100 * MB));
+        assert(fake::pinned.size() == 1 && fake::host_bytes <= (long)(30 * MB));
+        xfer_release();
+        assert(!fake::pinned.empty());
+        xfer_release();
+        assert(fake::pinned.empty());
+        const int n = fake::host_allocs;
+        for (int k = 0; k < 5; ++k) {       /* one handle after another */
+            xfer_retain();
+            assert(both(60 * MB));
+            xfer_release();
+        }
+        assert(fake::host_allocs == n);
+        xfer_retain();                      /* a large transfer in chunks: from the first on */
+        std::vector<unsigned char> a(60 * MB), dev(60 * MB);
+        XferSeg s = {a.data(), dev.data(), 60 * MB};
+        int stream = 0;
+        assert(xfer_up(&s, 1, 0, &stream, 500 * MB) == cudaSuccess && fake::host_allocs == n + 1);
+    } else if (what == "reset") {
+        /* pinned pieces that are gone (a reset device) are not written to */
+        assert(both(100 * MB));
+        for (void* p : std::set<void*>(fake::pinned)) cudaFreeHost(p);
         assert(both(100 * MB));
     } else if (what == "failing_copy") {
         assert(both(100 * MB));
@@ -124,7 +162,7 @@ def driver(tmp_path_factory):
 
 
 @pytest.mark.parametrize("what", ["bytes", "own_context", "no_primary", "capture", "no_pinned",
-                                  "failing_copy"])
+                                  "on_demand", "reset", "failing_copy"])
 def test_staged_copies(driver, what):
     r = subprocess.run([driver, what], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout == "ok\n", r.stderr
