@@ -384,9 +384,9 @@ ST_API int st_finalize(void);
  * and a call on a capturing stream is rejected with ST_ERR_INVALID_ARGUMENT before anything
  * is launched.  The first call on a device looks up the scratch array's address and keeps
  * it for the life of the process: do not call it on a device after cudaDeviceReset.  All
- * calls share the one array: calls that overlap on the GPU race.  Each call chooses its
- * fixed-point scale from its own deposits, so the source agrees with st_step's to the
- * fixed-point resolution and positions and velocities are bit-identical. */
+ * calls share the one array: calls that overlap on the GPU race (calls after them do not).
+ * Each call chooses its fixed-point scale from its own deposits, so the source agrees with
+ * st_step's to the fixed-point resolution and positions and velocities are bit-identical. */
 ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* mesh, int64_t n, double* x,
                            double* y, double* z, float* u, float* v, float* w, const float* d,
                            const float* U, double* source, double dt, double fluid_scale,

@@ -17,8 +17,8 @@
  * back and synchronising the stream, so a call cannot be recorded into a CUDA graph: one
  * made on a capturing stream is rejected before anything is launched.  All calls share the
  * one array and it keeps the last call's contents: each call clears the accumulator before
- * use and resets the control blocks of the call after it, and calls that overlap on the GPU
- * (other streams or host threads) race on the array.
+ * use and resets the control blocks of the call after it (st_turns.h), and calls that overlap on
+ * the GPU (other streams or host threads) race on the array; calls after them are sound again.
  */
 #include <algorithm>
 #include <climits>
@@ -29,6 +29,7 @@
 
 #include "scaletrack.h"
 #include "st_device.cuh"
+#include "st_turns.h"
 
 using namespace st;
 
@@ -39,7 +40,7 @@ constexpr int64_t NOALLOC_MAX_CELLS = ST_NOALLOC_MAX_CELLS;  /* include/scaletra
 static __device__ unsigned long long g_st_noalloc_acc[NOALLOC_MAX_CELLS * 3];
 
 /* Control blocks of the probe and the step, two sets used in turn: every call's last kernel
- * resets the set of the next call. */
+ * resets the set of the next call (st_turns.h). */
 struct CtlPair {
     CloudCtl probe, step;
 };
@@ -52,11 +53,26 @@ struct Scratch {
     CtlPair* ctl = nullptr;
     unsigned long long* acc = nullptr;
     int resident[2] = {0, 0};  /* step blocks that stay resident on the device: one substep, several */
-    int next = 0;        /* the control set of the next call */
-    bool dirty = false;  /* a call failed before its last kernel: both sets need a reset */
+    Turns turns;
 };
 std::mutex g_mu;
 Scratch g_scratch[MAX_DEVICES];
+
+/* One call's turn with the control sets of a device. */
+struct Call {
+    int dev;
+    Turns::Turn turn;
+    cudaStream_t s;
+    bool complete = false;   /* every kernel of the call has run */
+    Call(int device, const Turns::Turn& t, cudaStream_t stream) : dev(device), turn(t), s(stream) {}
+    Call(const Call&) = delete;
+    ~Call()
+    {
+        if (!complete) cudaStreamSynchronize(s);   /* what was launched before the failure */
+        std::lock_guard<std::mutex> lk(g_mu);
+        g_scratch[dev].turns.end(complete);
+    }
+};
 
 int fail(int code, const char* msg)
 {
@@ -165,6 +181,7 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
                         "CUDA graph");
     }
     Scratch sc;
+    Turns::Turn turn;
     {
         std::lock_guard<std::mutex> lk(g_mu);
         Scratch& g = g_scratch[dev];
@@ -183,12 +200,12 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
             g.acc = static_cast<unsigned long long*>(pa);
         }
         sc = g;
-        g.next ^= 1;
-        g.dirty = true;   /* until this call's last kernel is on its way */
+        turn = g.turns.begin();
     }
-    CtlPair* const ctl = sc.ctl + sc.next;
-    unsigned long long* const acc = sc.acc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    Call call(dev, turn, s);
+    CtlPair* const ctl = sc.ctl + turn.set;
+    unsigned long long* const acc = sc.acc;
     const int64_t ncomp = ncells * 3;
     const int64_t resident = sc.resident[p->n_substeps > 1];
 
@@ -232,7 +249,7 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
     a.one = ck;
 
     cudaError_t e;
-    if (sc.dirty) {
+    if (turn.reset) {
         k_noalloc_reset<<<1, 32, 0, s>>>(sc.ctl);
         if ((e = cudaGetLastError()) != cudaSuccess)
             return fail(ST_ERR_CUDA, cudaGetErrorString(e));
@@ -258,17 +275,14 @@ ST_API int st_step_noalloc(const st_params* p, const st_mesh_desc* m, int64_t n,
     }
     const int fgrid = (int)std::min<int64_t>((ncomp + 255) / 256, 148 * 8);
     e = launch_kernel(true, k_noalloc_finalize, dim3(fgrid), dim3(256), 0, s, acc, ctl,
-                      sc.ctl + (sc.next ^ 1), H, source, ncomp);
+                      sc.ctl + (turn.set ^ 1), H, source, ncomp);
     if (e != cudaSuccess) return fail(ST_ERR_CUDA, cudaGetErrorString(e));
-    {
-        std::lock_guard<std::mutex> lk(g_mu);
-        g_scratch[dev].dirty = false;
-    }
 
     CloudCtl out;
     if ((e = cudaMemcpyAsync(&out, &ctl->step, sizeof out, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return fail(ST_ERR_CUDA, cudaGetErrorString(e));
+    call.complete = true;
     if (out.lost) return fail(ST_ERR_PARCEL_OUTSIDE, "parcel(s) could not be located in the mesh");
     if (out.overflow)
         return fail(ST_ERR_SOURCE_RANGE, "deposit(s) exceeded the fixed-point range");
