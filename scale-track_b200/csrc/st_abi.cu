@@ -1277,37 +1277,45 @@ int adj_prepare(st_handle* h, int cloud, const st_adjoint_desc* d)
     const int64_t n = h->clouds[cloud].n;
     const int T = d->n_steps, C = d->checkpoint_interval;
     const int nseg = (T + C - 1) / C;
-    const int grid = adj_reverse_grid<P, V>(n, h->nsm);
+    int grid = adj_reverse_grid<P, V>(n, h->nsm);
+    const int width = adj_rec_width(n);
     const int limbs = sizeof(V) == 8 ? 2 : 1;
     size_t off = 0;
     auto carve = [&](size_t b) { size_t o = off; off += align256(b); return o; };
     const size_t o_ckx = carve((size_t)nseg * 3 * n * sizeof(P));
     const size_t o_ckv = carve((size_t)nseg * 3 * n * sizeof(V));
-    const size_t o_rec = carve((size_t)grid * C * 256 * adj_rec_bytes<V>);
-    const size_t o_y = carve((size_t)h->stride * sizeof(double));
     const size_t o_G = carve((size_t)h->stride * sizeof(V));
     const size_t o_dv = carve((size_t)3 * n * sizeof(double));
     const size_t o_pa = carve((size_t)((n + 255) / 256 + 1) * 2 * sizeof(double));
     const size_t o_fs = carve((size_t)2 * T * sizeof(V));   /* fs, then fs_lo */
+    /* the mean source of the forward pass, then the cotangent of the pull-back */
     const size_t o_mean = carve((size_t)h->stride * sizeof(double));
     const size_t o_ctl = carve(sizeof(CloudCtl));
     const size_t o_acc = carve((size_t)h->stride * limbs * 8);
+    const size_t o_rec = off, slot = (size_t)C * width * adj_rec_bytes<V>;
+    off += align256(grid * slot);
     if (off > t.bytes) {
         if (t.mem) cudaFree(t.mem);
         t.mem = nullptr;
         t.bytes = 0;
-        CK(cudaMalloc(&t.mem, off));
+        /* fewer blocks of the reverse kernel where their records do not fit */
+        cudaError_t e;
+        while ((e = cudaMalloc(&t.mem, off)) == cudaErrorMemoryAllocation && grid > 1) {
+            cudaGetLastError();
+            grid = (grid + 1) / 2;
+            off = o_rec + align256(grid * slot);
+        }
+        CK(e);
         t.bytes = off;
     }
     char* b = static_cast<char*>(t.mem);
     t.ck_x = b + o_ckx; t.ck_v = b + o_ckv;
     t.rec = reinterpret_cast<unsigned char*>(b + o_rec);
-    t.ybar = reinterpret_cast<double*>(b + o_y);
     t.G = b + o_G;
     t.dv0 = reinterpret_cast<double*>(b + o_dv);
     t.partials = reinterpret_cast<double*>(b + o_pa);
     t.fsd = b + o_fs;
-    t.mean = reinterpret_cast<double*>(b + o_mean);
+    t.mean = t.ybar = reinterpret_cast<double*>(b + o_mean);
     t.ctl = reinterpret_cast<CloudCtl*>(b + o_ctl);
     t.acc = reinterpret_cast<unsigned long long*>(b + o_acc);
     t.cloud = cloud; t.T = T; t.C = C; t.nseg = nseg; t.grid = grid; t.limbs = limbs;
@@ -1343,6 +1351,7 @@ AdjArgs<P, V> adj_args(st_handle* h)
     a.acc = t.acc; a.ctl = t.ctl;
     a.ck_x = (P*)t.ck_x; a.ck_v = (V*)t.ck_v;
     a.rec = t.rec;
+    a.width = adj_rec_width(t.n);
     a.G = (const V*)t.G;
     a.id = c.id[c.cur];
     a.dv0 = t.dv0;

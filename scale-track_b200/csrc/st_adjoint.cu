@@ -33,6 +33,7 @@
  * (records per parcel in HBM, power and cell velocity formed again in the reverse step before).
  */
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "st_step.cuh"
@@ -318,21 +319,24 @@ __global__ void __launch_bounds__(256) k_adj_forward(const AdjArgs<P, V> a)
 }
 
 /* The pull-back of 256 parcels at a time, all checkpoint segments from the last to the
- * first.  Records of a block: AdjRec[C][256], then cells int32[C][256] (-1: lost, below that
- * -2 - cell: bounced, flags in the bytes that follow), then flags uint8[C][256]. */
+ * first.  Records of a block, W = a.width: AdjRec[C][W], then cells int32[C][W] (-1: lost,
+ * below that -2 - cell: bounced, flags in the bytes that follow), then flags uint8[C][W].
+ * WIDE: the width is 256 as a constant; read from the arguments, in 64 bits, it takes 1 to 3 %
+ * longer (300000 FP64 parcels, 200 steps: 1.584 -> 1.636 ms). */
 /* Resident blocks: 3 (80 registers) in mixed precision, 4 in FP64 (3e5 parcels, 200 steps:
  * 1.83 ms with 3, 1.72 ms with 4). */
-template <class P, class V>
+template <class P, class V, bool WIDE>
 __global__ void __launch_bounds__(256, sizeof(V) == 8 ? 4 : 3) k_adj_reverse(const AdjArgs<P, V> a)
 {
     __shared__ double red[2][256];
     const int tid = threadIdx.x;
-    unsigned char* const slot = a.rec + (int64_t)blockIdx.x * a.C * 256 * adj_rec_bytes<V>;
+    const std::conditional_t<WIDE, int, int64_t> W = WIDE ? 256 : a.width;
+    unsigned char* const slot = a.rec + (int64_t)blockIdx.x * a.C * W * adj_rec_bytes<V>;
     AdjRec<V>* const rec = reinterpret_cast<AdjRec<V>*>(slot) + tid;
     int32_t* const rec_c =
-        reinterpret_cast<int32_t*>(slot + (int64_t)a.C * 256 * sizeof(AdjRec<V>)) + tid;
+        reinterpret_cast<int32_t*>(slot + (int64_t)a.C * W * sizeof(AdjRec<V>)) + tid;
     uint8_t* const rec_b =
-        slot + (int64_t)a.C * 256 * (sizeof(AdjRec<V>) + sizeof(int32_t)) + tid;
+        slot + (int64_t)a.C * W * (sizeof(AdjRec<V>) + sizeof(int32_t)) + tid;
     const int nseg = (a.T + a.C - 1) / a.C;
     const int64_t chunks = (a.n + 255) / 256;
     for (int64_t ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
@@ -364,22 +368,22 @@ __global__ void __launch_bounds__(256, sizeof(V) == 8 ? 4 : 3) k_adj_reverse(con
 #pragma unroll
                             for (int k = 0; k < 3; ++k) r.x[k] = o.du[k];
                         }
-                        rec[t * 256] = r;
-                        if (b) rec_b[t * 256] = (uint8_t)b;
+                        rec[t * W] = r;
+                        if (b) rec_b[t * W] = (uint8_t)b;
                     }
-                    rec_c[t * 256] = !ok ? -1 : (b ? -2 - cell : cell);
+                    rec_c[t * W] = !ok ? -1 : (b ? -2 - cell : cell);
                 }
-                int32_t cn = rec_c[(len - 1) * 256];
-                AdjRec<V> rn = rec[(len - 1) * 256];
+                int32_t cn = rec_c[(len - 1) * W];
+                AdjRec<V> rn = rec[(len - 1) * W];
                 for (int t = len - 1; t >= 0; --t) {  /* reverse, the next record in flight */
                     const int32_t cc = cn;
                     const AdjRec<V> r = rn;
                     if (t > 0) {
-                        cn = rec_c[(t - 1) * 256];
-                        rn = rec[(t - 1) * 256];
+                        cn = rec_c[(t - 1) * W];
+                        rn = rec[(t - 1) * W];
                     }
                     if (cc == -1) continue;
-                    const unsigned b = cc < 0 ? rec_b[t * 256] : 0u;
+                    const unsigned b = cc < 0 ? rec_b[t * W] : 0u;
                     adj_reverse<P, V>(a, q, r, a.fs[n0 + t], a.fs_lo[n0 + t],
                                       cc < 0 ? -2 - cc : cc, b, av, dalpha, dscale);
                 }
@@ -461,7 +465,9 @@ template <class P, class V>
 cudaError_t launch_adj_reverse(const AdjArgs<P, V>& a, int grid, cudaStream_t s)
 {
     if (grid == 0) return cudaSuccess;
-    k_adj_reverse<P, V><<<grid, 256, 0, s>>>(a);
+    /* the record indices of a block are below 256 * C */
+    if (a.width == 256 && a.C < INT32_MAX / 256) k_adj_reverse<P, V, true><<<grid, 256, 0, s>>>(a);
+    else k_adj_reverse<P, V, false><<<grid, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -470,7 +476,7 @@ template <class P, class V>
 int adj_reverse_grid(int64_t n, int nsm)
 {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_adj_reverse<P, V>, 256, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_adj_reverse<P, V, true>, 256, 0) !=
             cudaSuccess || nb < 1)
         nb = 1;
     const int64_t chunks = (n + 255) / 256;

@@ -240,7 +240,8 @@ struct AdjArgs {
     CloudCtl* ctl;              /* scale and counters of the adjoint run */
     P* ck_x;                    /* checkpoints [nseg][3][n] */
     V* ck_v;
-    unsigned char* rec;         /* records of one segment, [reverse grid][C * 256 * rec bytes] */
+    unsigned char* rec;         /* records of one segment, [reverse grid][C * width * rec bytes] */
+    int width;                  /* parcels that a block records (adj_rec_width) */
     const V* G;                 /* dJ/dS_n per cell component [ncomp] */
     const int32_t* id;          /* st_set_parcels index of each parcel */
     double* dv0;                /* velocity cotangent [3][n] by that index, or null */
@@ -250,6 +251,9 @@ struct AdjArgs {
 /* Bytes of a reverse record: four V, the cell, the bounce flags. */
 template <class V>
 constexpr int adj_rec_bytes = 4 * sizeof(V) + sizeof(int32_t) + 1;
+/* Parcels whose records a reverse block holds: its 256 threads', fewer with fewer parcels (one
+ * block then; a multiple of 32 keeps the records aligned). */
+inline int adj_rec_width(int64_t n) { return n >= 256 ? 256 : (int)((n + 31) / 32 * 32); }
 
 template <class P, class V>
 cudaError_t launch_adj_forward(const AdjArgs<P, V>& a, bool probe, cudaStream_t s);
