@@ -764,19 +764,29 @@ constexpr int64_t PARCEL_CHUNK = (int64_t)1 << 20;
 
 int64_t even(int64_t n) { return n + (n & 1); }
 
+/* Small clouds hold every parcel array in room for doubles (1.5 MB more at most), so that all
+ * parcels are staged at once: each chunk costs seven copies of about 10 us (2075 mixed parcels
+ * read back after four steps: 262 us in two chunks, 185 in one). */
+bool small_cloud(int64_t cap) { return cap * 7 * (int64_t)sizeof(double) < ((int64_t)2 << 20); }
+
+size_t parcel_array_bytes(int64_t cap, size_t elem)
+{
+    return (size_t)cap * (small_cloud(cap) ? sizeof(double) : elem);
+}
+
 /* Where the chunks of m parcels are staged, in the caller's doubles, and how many at a time.  In
  * the cloud's idle buffers (c.x[1 - cur] ..., free between steps), which takes no memory: an
  * array of cap floats holds cap / 2 doubles, and cap is even.  Where that would cut a large
  * transfer into more chunks, the handle's staging array instead (at most 59 MB), if there is
  * memory for it: 1e6 FP32 parcels read back in one chunk 2.57 ms, in two 2.95 ms; a small cloud
- * set without the allocation 0.57 -> 0.47 ms. */
+ * set without that allocation 0.57 -> 0.46 ms. */
 template <class V>
 int64_t parcel_stage(st_handle* h, const CloudBufs& c, int64_t m, ParcelStage& st)
 {
     const int64_t want = std::min(m, PARCEL_CHUNK);
-    const int64_t idle = c.cap * (int64_t)sizeof(V) / (int64_t)sizeof(double);
-    const size_t bytes = (size_t)want * 7 * sizeof(double);
-    if (idle < want && bytes >= ((size_t)2 << 20) && try_stage(h, bytes)) {
+    const int64_t idle =
+        small_cloud(c.cap) ? c.cap : c.cap * (int64_t)sizeof(V) / (int64_t)sizeof(double);
+    if (idle < want && try_stage(h, (size_t)want * 7 * sizeof(double))) {
         double* const p = static_cast<double*>(h->dstage);
         st = {p, p + want, p + 2 * want, p + 3 * want, p + 4 * want, p + 5 * want, p + 6 * want};
         return want;
@@ -833,7 +843,7 @@ int do_set_parcels(st_handle* h, int cloud, int64_t n, const double* xyz, const 
             for (int a = 0; a < 7; ++a) {
                 if (*arrs[a]) cudaFree(*arrs[a]);
                 *arrs[a] = nullptr;
-                CK(cudaMalloc(arrs[a], (size_t)cap * (a < 3 ? sizeof(P) : sizeof(V))));
+                CK(cudaMalloc(arrs[a], parcel_array_bytes(cap, a < 3 ? sizeof(P) : sizeof(V))));
             }
             if (c.id[k]) cudaFree(c.id[k]);
             if (c.keys[k]) cudaFree(c.keys[k]);
@@ -943,7 +953,9 @@ int do_append_parcels(st_handle* h, int cloud, int64_t m, const double* xyz, con
         void* nperm[2];
         bool ok = true;
         for (int k = 0; k < 2 && ok; ++k) {
-            for (int a = 0; a < 8 && ok; ++a) ok = (nb[k][a] = grab((size_t)cap * es[a])) != nullptr;
+            for (int a = 0; a < 8 && ok; ++a)
+                ok = (nb[k][a] = grab(a < 7 ? parcel_array_bytes(cap, es[a])
+                                            : (size_t)cap * es[a])) != nullptr;
             ok = ok && (nkeys[k] = grab((size_t)cap * sizeof(uint32_t))) != nullptr;
             ok = ok && (nperm[k] = grab((size_t)cap * sizeof(uint32_t))) != nullptr;
         }
