@@ -525,12 +525,18 @@ bool use_pdl(const st_handle* h)
  *   hex, FP32 and mixed:  1e4 15.9 / 9.5   1e5 14.6 / 12.3   1.5e6 41.1 / 41.0   4e6 84.5 / 92.6
  *   hex, FP64:   1e5 17.7 / 15.0   4e5 25.2 / 24.9   5e5 30.1 / 32.1   4e6 141 / 151
  *   hex, mixed, ten substeps:  1e6 118 / 99   4e6 386 / 333   1e7 987 / 859
- * On larger meshes the conversion weighs more, and the ring's overlapped one pays earlier (two
- * steps, three handles in turn):
- *   mixed, 76^3:  1e5 29.8 / 40.7   1e6 65.8 / 76.9;  128^3:  1e5 65.5 / 79.5   1e6 136 / 149
- *   mixed, 90^3:  2e4 32.5 / 28.2;  FP64, 60^3:  1e5 30.9 / 35.5;  100^3:  1e5 61.8 / 74.7
- *   mixed, 60^3:  1e5 28.1 / 24.3   3e5 28.1 / 29.6   7e5 46.3 / 49.6
- *   mixed, 48^3:  3e5 26.2 / 23.4   1.3e6 63.5 / 61.8;  FP64, 48^3:  3e5 35.1 / 33.4
+ * On larger meshes the conversion weighs more, and the ring hides more of it (deterministic
+ * deposit, two steps, one handle, the per-warp kernel's conversion overlapped as the ring's where
+ * launches are plain, as do_step chooses):
+ *   mixed, 60^3:  1e5 43.9 / 45.3   76^3:  5e4 54.5 / 47.7   1e5 55.0 / 55.4   1e6 90.0 / 87.5
+ *   mixed, 100^3:  1e5 76.1 / 86.3;  128^3:  1e5 111.9 / 122.7   1e6 176.5 / 182.8
+ *   mixed, 48^3:  3e5 43.6 / 42.6;  32^3:  4e5 47.9 / 43.7;  64^3:  1e6 80.3 / 75.6   4e6 182 / 199
+ *   FP64, 60^3:  1e5 50.7 / 47.2;  76^3:  1e5 60.4 / 57.2   1e6 119 / 124;  100^3:  1e5 80.0 / 87.4
+ * and with three handles in turn, whose passes overlap on the GPU: mixed, 76^3:  1e5 29.8 / 40.7
+ * 1e6 65.8 / 76.9;  60^3:  3e5 28.1 / 29.6;  FP64, 60^3:  1e5 30.9 / 35.5.  The atomic deposit
+ * converts nothing, and the mesh does not count (two steps, one handle):
+ *   atomic, mixed, 76^3:  1e5 46.4 / 36.2   1e6 76.6 / 76.7;  128^3:  1e5 85.8 / 70.3   1e6 124 / 119
+ *   atomic, FP64, 32^3:  4e5 41.9 / 40.1;  76^3:  5e4 47.2 / 31.7   1e6 89 / 101;  128^3:  1e6 136 / 158
  *   tet, mixed:  2e5 22.0 / 20.4   4e5 27.1 / 27.6   1e6 43.6 / 46.2; three substeps: 1e6 73 / 78
  *   tet, FP64:   4e5 33.6 / 35.3   1e6 75.2 / 79.4   2e6 123 / 131
  * A wait limit set by the caller is about the ring's waits: the ring then runs at any size. */
@@ -541,8 +547,10 @@ bool use_ring(const st_handle* h, int64_t n)
     const bool fp64 = h->p.precision == ST_PREC_FP64;
     if (h->tet) return n >= 300000;
     if (h->p.n_substeps != 1) return false;
-    if (acc_bytes(h) > PDL_BYTES && n >= 50000) return true;
-    if (h->stride >= 3 * 200000 && n >= 250000) return true;
+    if (h->dep != DEP_ATOMIC) {
+        if (acc_bytes(h) > PDL_BYTES && n >= 50000) return true;
+        if (h->stride >= 3 * 200000 && n >= 250000) return true;
+    }
     return n >= (fp64 ? 450000 : 1500000);
 }
 

@@ -94,3 +94,22 @@ def test_one_handle_across_the_rules(prec, mesh, counts):
                 h.append_parcels(*[a[..., :m] for a in sets[1]])
                 steps(h, 3)
                 assert np.array_equal(grown, h.get_source())
+
+
+def test_atomic_deposit_across_the_rules():
+    """On a mesh whose accumulators would be above 8 MB; the sums within 1e-12 of the per-warp
+    kernel's (a cell's few deposits in another order: some 2^-53 of the sum of magnitudes)."""
+    U = workload.tgv_field(72, dtype=np.float64)
+    for n in (60_000, 440_000, 460_000):
+        p = workload.parcels(n, 310)
+        out = []
+        for kind in (None, "warp"):
+            with handle("fp64", 72, deposit="atomic") as h:
+                if kind:
+                    h.set_step_kernel(kind)
+                h.set_fluid_velocity(U)
+                h.set_parcels(*p)
+                steps(h, 3)
+                out.append((h.get_source(), h.get_parcels()[0]))
+        assert np.array_equal(out[0][1], out[1][1])
+        assert np.abs(out[0][0] - out[1][0]).max() <= 1e-12 * np.abs(out[1][0]).max()
