@@ -504,7 +504,9 @@ int do_sort_all(st_handle* h)
  * Beyond, the blocks that wait take SMs from other handles' steps (three handles in turn, with
  * and without: 14 clouds, 15 MB, two steps 41 and 35 us; 20 FP64 clouds, 23 MB, 121 and 108; one
  * cloud of 4e6 parcels, 4 MB, two times ten substeps 650 and 597; 2.5e5 parcels, 0.4 MB, 64 and
- * 68). */
+ * 68).  A handle alone gains beyond the lines too (two steps, with and as the rule has it:
+ * 1.3e6 parcels on 48^3 cells 72.6 and 75.3 us, 3e4 on 100^3 42.6 and 48.2; 14 clouds on 36^3
+ * 62.2 and 69.9): the lines are drawn for programs with several. */
 constexpr size_t PDL_BYTES = (size_t)8 << 20;
 constexpr int64_t PDL_PARCELS = 500000;
 

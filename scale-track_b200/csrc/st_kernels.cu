@@ -410,7 +410,11 @@ __global__ void __launch_bounds__(256) k_finalize(unsigned long long* __restrict
  * pass of two steps; 403 MB: 1207 against 1386 us; one cloud on 1.6e6 tets, 38 MB: 62.6 against
  * 66 us).  Between, where the accumulators of many clouds fit the L2 but not along with all
  * else, they are read evict-first and a memset of its own leaves their zeros in the L2 for the
- * step's adds (33 MB: 145 against 165 us; 36 MB: 84 against 90; 84 MB: 217 against 220). */
+ * step's adds (three handles in turn, by the memset and by the conversion: 33 MB 145 and 165 us;
+ * 36 MB 84 and 90; 84 MB 217 and 220).  One handle alone is faster with the conversion there too
+ * (64^3 cells, two steps: 31 MB 75.5 and 53.9 us, 82 MB 150 and 125; 50 MB in FP64 88.9 and 63.4):
+ * the lines are drawn for programs with several handles.  Outside them both agree on the
+ * conversion (19 MB 60.2 and 47.6 us; 126 MB 217 and 204). */
 cudaError_t launch_finalize(int limbs, unsigned long long* acc, double* src, float* src32,
                             CloudCtl* ctl, const int32_t* Lsrc, unsigned int* counter,
                             int nclouds, int64_t stride, int grid_x, cudaStream_t s, bool pdl)
