@@ -735,6 +735,7 @@ int do_step_tet(st_handle* h, double dt, double fscale, int phase)
     if (!h->capturing && h->clouds_dirty && (rc = upload_clouds<double, V>(h)) != ST_OK) return rc;
     TetStepArgs<V> a;
     a.mesh = h->tmesh;
+    a.mesh.sorted = h->p.sort_interval > 0;
     a.phys = phys_k<V>(h);
     a.dtP = dt / (double)h->p.n_substeps;
     a.dtV = (V)a.dtP;
@@ -1659,7 +1660,7 @@ static int create_impl(const st_params* p, const st_mesh_desc* m, int64_t ncells
         float xf = (float)xm;
         if ((double)xf < xm) xf = std::nextafter(xf, INFINITY);
         k.xmax = xf;
-        k.pad0 = 0;
+        k.sorted = 0;
         k.hop_limit = tm->hop_limit > 0 ? tm->hop_limit : 64;
         k.pad = 0;
     }

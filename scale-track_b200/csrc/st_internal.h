@@ -165,7 +165,7 @@ struct TetMeshK {
     const double4* planes;      /* [nt][4] outward face planes (n0, n1, n2, c), s = n.x - c */
     const float4* planes32;     /* the same planes rounded to FP32 (the walk's pre-check) */
     float xmax;                 /* max |coordinate| of any point of the box, rounded up */
-    int32_t pad0;
+    int32_t sorted;             /* the cloud is re-sorted by tet (ring kernel: tet_walk) */
     const int32_t* nbr;         /* [nt][4] tet across the face opposite local vertex k, or -1 */
     int64_t nt;
     double origin[3];

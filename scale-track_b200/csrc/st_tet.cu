@@ -150,7 +150,17 @@ __device__ __forceinline__ int tet_step32(const TetMeshK& m, int32_t t, const fl
 }
 
 /* Greedy walk; at most hop_limit moves (bounded loop).  Each step is decided in FP32 where
- * tet_step32 can, else from the FP64 planes; both give the FP64 walk's tets and hops. */
+ * tet_step32 can, else from the FP64 planes; both give the FP64 walk's tets and hops.
+ *
+ * BESIDE: all four neighbours are loaded beside the planes, so that a hop waits for one load,
+ * not two.  That pays where the parcels are re-sorted by tet and neighbouring lanes share the
+ * lines (mixed precision, 2e7 parcels on 5.3e6 tets, a re-sort every ten steps: 623 us per launch,
+ * 642 with one neighbour loaded once it is known which); not where they are not, as every look,
+ * also the ones that end a walk, reads 16 bytes more (5e6 unsorted parcels on 1.6e6 tets: 365 us
+ * beside the planes, 281 alone), and not with FP64 velocities, whose steps wait less on the walk
+ * (sorted 242 and 237 us, unsorted 532 and 486).  An instance each: chosen by a flag inside the
+ * walk, the sorted step took 638 us. */
+template <bool BESIDE>
 __device__ __forceinline__ int32_t tet_walk(const TetMeshK& m, int32_t t, const double x[3],
                                             int hop_limit, int& status, int& hops)
 {
@@ -162,6 +172,8 @@ __device__ __forceinline__ int32_t tet_walk(const TetMeshK& m, int32_t t, const 
                      fabs(x[2]) <= (double)m.xmax;
     for (int it = 0; it <= hop_limit; ++it) {
         int fb = 0;
+        int4 nbr;
+        if constexpr (BESIDE) nbr = __ldg(reinterpret_cast<const int4*>(m.nbr) + t);
         const int r = pre ? tet_step32(m, t, x32, fb) : 0;
         if (r == 1) {
             status = TWALK_OK;
@@ -179,10 +191,9 @@ __device__ __forceinline__ int32_t tet_walk(const TetMeshK& m, int32_t t, const 
                 return t;
             }
         }
-        /* one neighbour, once it is known which: all four beside the planes read 16 bytes more on
-         * every look, also of the walks that end there (5e6 unsorted parcels on 1.6e6 tets: 365
-         * us per launch beside the planes, 281 now; sorted 145 and 148) */
-        const int32_t nb = __ldg(m.nbr + 4 * (int64_t)t + fb);
+        int32_t nb;
+        if constexpr (BESIDE) nb = fb == 0 ? nbr.x : (fb == 1 ? nbr.y : (fb == 2 ? nbr.z : nbr.w));
+        else nb = __ldg(m.nbr + 4 * (int64_t)t + fb);
         if (nb < 0) {
             status = TWALK_EXIT;
             return t;
@@ -216,7 +227,7 @@ __shared__ unsigned s_tet_hist[8];
  * the final deposit is returned in (key, dep) for the warp reduction, intermediate deposits
  * (substeps > 1) go straight to memory.  With count_hops, walk lengths go to the block's
  * histogram s_tet_hist. */
-template <class V, int DEP>
+template <class V, int DEP, bool BESIDE>
 __device__ __forceinline__ void tet_parcel(const TetStepArgs<V>& a, int nsub, double pos[3],
                                            V vel[3], V d, int32_t& cell,
                                            unsigned long long* acc, double* src,
@@ -283,7 +294,7 @@ __device__ __forceinline__ void tet_parcel(const TetStepArgs<V>& a, int nsub, do
             }
         }
         int status = TWALK_OK, hops = 0;
-        tNew = tet_walk(a.mesh, tNew, posNew, a.mesh.hop_limit, status, hops);
+        tNew = tet_walk<BESIDE>(a.mesh, tNew, posNew, a.mesh.hop_limit, status, hops);
         if (status != TWALK_OK) { lost = true; break; }
         if (count_hops) atomicAdd(&s_tet_hist[hops < 7 ? hops : 7], 1u);
         if (t != nsub && tNew != cur) {
@@ -381,7 +392,7 @@ __global__ void __launch_bounds__(256, TetMinBlocks<V>::value) k_step_tet(const 
              * now, alongside the cell-velocity gather */
             asm volatile("prefetch.global.L1 [%0];" ::"l"(a.mesh.planes32 + 4 * (int64_t)cell));
             bool lost = false;
-            tet_parcel<V, DEP>(a, nsub, pos, vel, d, cell, acc, src, qp, amax, ovf, lost, key,
+            tet_parcel<V, DEP, false>(a, nsub, pos, vel, d, cell, acc, src, qp, amax, ovf, lost, key,
                                dep, count_hops);
             if (lost) {
                 ++nlost;
@@ -421,7 +432,7 @@ using TetShape = RingShape<992, 31>;
 
 /* The consumer work of the tet ring: each warp's slices of 32 parcels through
  * tet_parcel, the new state written back into the tile, deposits reduced per slice. */
-template <class V, int DEP, bool ONE>
+template <class V, int DEP, bool ONE, bool BESIDE>
 struct TetRing {
     const TetStepArgs<V>& a;
     unsigned long long* acc;
@@ -452,7 +463,7 @@ struct TetRing {
                 /* the walk's first planes, alongside the cell-velocity gather */
                 asm volatile("prefetch.global.L1 [%0];" ::"l"(a.mesh.planes32 + 4 * (int64_t)cell));
                 bool lost = false;
-                tet_parcel<V, DEP>(a, nsub, pos, vel, d, cell, acc, src, qp, amax, ovf, lost,
+                tet_parcel<V, DEP, BESIDE>(a, nsub, pos, vel, d, cell, acc, src, qp, amax, ovf, lost,
                                    key, dep, count_hops);
                 if (lost) {
                     ++nlost;
@@ -472,7 +483,7 @@ struct TetRing {
     }
 };
 
-template <class V, int DEP, bool ONE>
+template <class V, int DEP, bool ONE, bool BESIDE>
 __global__ void __launch_bounds__(TetShape::THREADS, 1) k_step_tet_ring(const TetStepArgs<V> a)
 {
     constexpr bool DET = (DEP == DEP_DET1 || DEP == DEP_DET2);
@@ -487,7 +498,7 @@ __global__ void __launch_bounds__(TetShape::THREADS, 1) k_step_tet_ring(const Te
     if (threadIdx.x < 8) s_tet_hist[threadIdx.x] = 0;   /* ring_block synchronises */
     ring_emax_init();
     __shared__ __align__(16) unsigned long long dep_ws[TetShape::CONS][dep_ws_words<DEP, V>];
-    TetRing<V, DEP, ONE> step{a, DET ? a.one.acc : nullptr,
+    TetRing<V, DEP, ONE, BESIDE> step{a, DET ? a.one.acc : nullptr,
                               DEP == DEP_ATOMIC ? a.one.src : nullptr, qp, lane, count_hops,
                               amax, ovf, nlost,
                               dep_ws[min(threadIdx.x >> 5, TetShape::CONS - 1)]};
@@ -501,7 +512,7 @@ __global__ void __launch_bounds__(TetShape::THREADS, 1) k_step_tet_ring(const Te
         atomicMax(&a.ctl->emax, s_ring_emax);
 }
 
-template <class V, int DEP, bool ONE>
+template <class V, int DEP, bool ONE, bool BESIDE>
 static cudaError_t tet_ring_attr()
 {
     static std::atomic<unsigned long long> ready{0};
@@ -510,23 +521,35 @@ static cudaError_t tet_ring_attr()
     if (e != cudaSuccess) return e;
     const unsigned long long bit = 1ULL << (dev & 63);
     if (ready.load() & bit) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_step_tet_ring<V, DEP, ONE>,
+    e = cudaFuncSetAttribute(k_step_tet_ring<V, DEP, ONE, BESIDE>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)RingGeom<TetShape, double, V, true>::SMEM);
     if (e == cudaSuccess) ready.fetch_or(bit);
     return e;
 }
 
-template <class V, int DEP, bool ONE>
-static cudaError_t launch_tet_ring_t(const TetStepArgs<V>& a, int nsm, cudaStream_t s, bool pdl)
+template <class V, int DEP, bool ONE, bool BESIDE>
+static cudaError_t launch_tet_ring_i(const TetStepArgs<V>& a, int nsm, cudaStream_t s, bool pdl)
 {
-    cudaError_t e = tet_ring_attr<V, DEP, ONE>();
+    cudaError_t e = tet_ring_attr<V, DEP, ONE, BESIDE>();
     if (e != cudaSuccess) return e;
     const int64_t nfull = a.one.n / TetShape::BT;
     int64_t grid = nfull < nsm ? nfull : nsm;
     if (grid < 1) grid = 1;
-    return launch_kernel(pdl, k_step_tet_ring<V, DEP, ONE>, (int)grid, TetShape::THREADS,
+    return launch_kernel(pdl, k_step_tet_ring<V, DEP, ONE, BESIDE>, (int)grid, TetShape::THREADS,
                          RingGeom<TetShape, double, V, true>::SMEM, s, a);
+}
+
+/* Neighbours beside the planes (tet_walk): re-sorted clouds with FP32 velocities. */
+template <class V>
+constexpr bool tet_beside = sizeof(V) == 4;
+
+template <class V, int DEP, bool ONE>
+static cudaError_t launch_tet_ring_t(const TetStepArgs<V>& a, int nsm, cudaStream_t s, bool pdl)
+{
+    if (tet_beside<V> && a.mesh.sorted)
+        return launch_tet_ring_i<V, DEP, ONE, tet_beside<V>>(a, nsm, s, pdl);
+    return launch_tet_ring_i<V, DEP, ONE, false>(a, nsm, s, pdl);
 }
 
 template <class V>
@@ -560,9 +583,14 @@ template <class V>
 cudaError_t tet_ring_prepare()
 {
     constexpr int DET = det_mode<V>;
-    const cudaError_t r[4] = {tet_ring_attr<V, DET, true>(), tet_ring_attr<V, DET, false>(),
-                              tet_ring_attr<V, DEP_ATOMIC, true>(),
-                              tet_ring_attr<V, DEP_ATOMIC, false>()};
+    constexpr bool B = tet_beside<V>;
+    const cudaError_t r[8] = {tet_ring_attr<V, DET, true, false>(),
+                              tet_ring_attr<V, DET, false, false>(),
+                              tet_ring_attr<V, DEP_ATOMIC, true, false>(),
+                              tet_ring_attr<V, DEP_ATOMIC, false, false>(),
+                              tet_ring_attr<V, DET, true, B>(), tet_ring_attr<V, DET, false, B>(),
+                              tet_ring_attr<V, DEP_ATOMIC, true, B>(),
+                              tet_ring_attr<V, DEP_ATOMIC, false, B>()};
     for (cudaError_t e : r)
         if (e != cudaSuccess) return e;
     return cudaSuccess;
@@ -628,7 +656,7 @@ __global__ void k_tet_locate(const TetMeshK m, const double* __restrict__ x,
         int32_t h = hint[i];
         int status = TWALK_EXIT, hops = 0;
         int32_t t = -1;
-        if (h >= 0 && h < m.nt) t = tet_walk(m, h, p, m.hop_limit, status, hops);
+        if (h >= 0 && h < m.nt) t = tet_walk<false>(m, h, p, m.hop_limit, status, hops);
         const bool ok = status == TWALK_OK;
         cells[i] = ok ? t : -1;
         if (!ok) atomicAdd(outside, 1ULL);
