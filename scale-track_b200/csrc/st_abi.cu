@@ -785,23 +785,24 @@ size_t parcel_array_bytes(int64_t cap, size_t elem)
     return (size_t)cap * (small_cloud(cap) ? sizeof(double) : elem);
 }
 
-/* Where the chunks of m parcels are staged, in the caller's doubles, and how many at a time.  In
- * the cloud's idle buffers (c.x[1 - cur] ..., free between steps), which takes no memory: an
- * array of cap floats holds cap / 2 doubles, and cap is even.  Where that would cut a large
- * transfer into more chunks, the handle's staging array instead (at most 59 MB), if there is
- * memory for it: 1e6 FP32 parcels read back in one chunk 2.57 ms, in two 2.95 ms; a small cloud
- * set without that allocation 0.57 -> 0.46 ms. */
+/* Where the chunks of m parcels are staged, in the caller's doubles, and how many at a time.
+ * Those of a small cloud in its idle buffers (c.x[1 - cur] ..., free between steps), which takes
+ * no memory: a handle of 1e4 parcels is set in 0.46 ms, with a staging array of its own 0.57 ms.
+ * Larger ones in the handle's staging array (at most 59 MB, which a conversion of U uses as
+ * well), in chunks as large as it is: 1e6 FP32 parcels read back in one chunk 2.57 ms, in the two
+ * that the idle buffers take 2.95 ms (an array of cap floats holds cap / 2 doubles; cap is even).
+ * Where there is no memory for it, in the idle buffers too. */
 template <class V>
 int64_t parcel_stage(st_handle* h, const CloudBufs& c, int64_t m, ParcelStage& st)
 {
     const int64_t want = std::min(m, PARCEL_CHUNK);
-    const int64_t idle =
-        small_cloud(c.cap) ? c.cap : c.cap * (int64_t)sizeof(V) / (int64_t)sizeof(double);
-    if (idle < want && try_stage(h, (size_t)want * 7 * sizeof(double))) {
+    const bool small = small_cloud(c.cap);
+    if (!small && try_stage(h, (size_t)want * 7 * sizeof(double))) {
         double* const p = static_cast<double*>(h->dstage);
         st = {p, p + want, p + 2 * want, p + 3 * want, p + 4 * want, p + 5 * want, p + 6 * want};
         return want;
     }
+    const int64_t idle = small ? c.cap : c.cap * (int64_t)sizeof(V) / (int64_t)sizeof(double);
     const int i = 1 - c.cur;
     st = {(double*)c.x[i], (double*)c.y[i], (double*)c.z[i], (double*)c.u[i],
           (double*)c.v[i], (double*)c.w[i], (double*)c.d[i]};

@@ -15,14 +15,16 @@
  * The staging buffer belongs to the process: a pinned piece for each thread that a copy has work
  * for, at most XFER_THREADS (24 MB), made when a copy first needs it and freed with the last
  * handle.  Pinning is dear (16 ms for 24 MB, 2.5 ms to free), so copies go through plain
- * cudaMemcpyAsync until XFER_RENT bytes have been copied, by when the staged copies would have
- * saved about as much (0.04 ms per MB up, 0.16 down into pages that are used again).  So a
- * program of small copies, or of one handle after another, does not pay for it each time (a fresh
- * handle's 1e5 FP64 parcels set 23 ms when the first copy of 2 MB made the buffer, 3.0 ms now, the
- * handle destroyed 5.9 and 2.8 ms; 1e6 FP32 parcels 28 and 12 ms, 11.5 and 7.7 ms).  One copy
- * uses the buffer at a time; a copy that finds it taken (another host thread's), or cannot have
- * it, and copies to pinned memory or below XFER_MIN, go through plain cudaMemcpyAsync, and so do
- * those of a handle in a context other than the device's primary one.
+ * cudaMemcpyAsync until XFER_RENT bytes have been copied: a program of small copies, or of one
+ * small handle after another, does not pay for it each time (a fresh handle's 1e5 FP64 parcels set
+ * 23 ms when the first copy of 2 MB made the buffer, 3.0 ms now, the handle destroyed 5.9 and
+ * 2.8 ms).  Staging earns 0.04 ms per MB up and 0.16 down into pages that are used again, so a
+ * later line (128 MB) suits fresh handles of 1e6 parcels in turn (set 12 ms, 28 with this line), and
+ * a program with more to copy pays for it then, in a pass (1e6 parcels' first adjoint pass on a
+ * fresh handle 27 to 35 ms, 11 with this line).  One copy uses the buffer at a time; a copy that
+ * finds it taken (another host thread's), or cannot have it, and copies to pinned memory or below
+ * XFER_MIN, go through plain cudaMemcpyAsync, and so do those of a handle in a context other than
+ * the device's primary one.
  */
 #include <algorithm>
 #include <atomic>
@@ -44,7 +46,7 @@ namespace {
  * sixteen 3.74 ms. */
 constexpr size_t XFER_PIECE = (size_t)2 << 20;
 constexpr size_t XFER_MIN = (size_t)2 << 20;
-constexpr size_t XFER_RENT = (size_t)128 << 20;
+constexpr size_t XFER_RENT = (size_t)48 << 20;
 constexpr int XFER_THREADS = 12;
 
 std::mutex g_users_mu;

@@ -93,11 +93,11 @@ int main(int argc, char** argv)
         fake::refuse_alloc = true;
         assert(both(300 * MB));
     } else if (what == "on_demand") {
-        /* nothing is pinned for small copies, or before 128 MB have been copied; then only what
+        /* nothing is pinned for small copies, or before 48 MB have been copied; then only what
          * the copy's threads use, at most 24 MB; and all of it goes with the last handle */
         for (int k = 0; k < 200; ++k) assert(both(2 * MB - 1));
         assert(fake::host_allocs == 0);
-        for (int k = 0; k < 12; ++k) assert(both(5 * MB));
+        for (int k = 0; k < 4; ++k) assert(both(5 * MB));
         assert(fake::host_allocs == 0);
         for (int k = 0; k < 5; ++k) assert(both(5 * MB));
         assert(fake::host_bytes > 0 && fake::host_bytes <= (long)(6 * MB));
@@ -111,13 +111,13 @@ int main(int argc, char** argv)
         const int n = fake::host_allocs;
         for (int k = 0; k < 5; ++k) {       /* one handle after another */
             xfer_retain();
-            assert(both(60 * MB));
+            assert(both(20 * MB));
             xfer_release();
         }
         assert(fake::host_allocs == n);
         xfer_retain();                      /* a large transfer in chunks: from the first on */
-        std::vector<unsigned char> a(60 * MB), dev(60 * MB);
-        XferSeg s = {a.data(), dev.data(), 60 * MB};
+        std::vector<unsigned char> a(30 * MB), dev(30 * MB);
+        XferSeg s = {a.data(), dev.data(), 30 * MB};
         int stream = 0;
         assert(xfer_up(&s, 1, 0, &stream, 500 * MB) == cudaSuccess && fake::host_allocs == n + 1);
     } else if (what == "reset") {
