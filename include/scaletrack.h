@@ -235,8 +235,8 @@ ST_API int st_autotune(st_handle* h, double dt, int trial_steps, st_tune_result*
 /* Step kernel of a handle with one cloud (cuboid or tet mesh).  ST_STEP_KERNEL_RING: a
  * persistent block per SM streams block tiles of about a thousand parcels through a
  * shared-memory ring with bulk copies.  ST_STEP_KERNEL_WARP: every warp loads and steps its
- * own 32 parcels.  Without this call the library takes the faster one for the cloud's size,
- * precision and substeps (the ring for large clouds).  Both give bit-identical positions,
+ * own 32 parcels.  Without this call the library takes the faster one for the cloud's size and mesh,
+ * precision, deposit and substeps (the ring for large clouds).  Both give bit-identical positions,
  * velocities, cells, sources and walk lengths; handles with several clouds, and the first
  * (probe) pass of a run, always use the warp kernel.  No counterpart in the
  * reference (one kernel, A:1258-1269). */
